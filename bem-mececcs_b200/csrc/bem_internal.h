@@ -81,6 +81,7 @@ constexpr int kPermStride = 1 + 2 * 128;
 struct LuWork {
   int cap_nn = 0, cap_batch = 0;
   int cluster_cs = 0;           // CTAs per panel cluster (16 or 8)
+  double2* panel_u = nullptr;   // [batch][64][64] U of a panel while it is factored in slices
   int* ipiv = nullptr;          // [batch][nn] 1-based pivot rows
   int* perm = nullptr;          // [panel][batch][kPermStride]
   std::vector<std::pair<int, int>> panels;  // (k, w) of every panel of the last factorisation

@@ -207,6 +207,7 @@ int bem_ctx_destroy(bem_ctx* ctx) {
   LuWork& L = ctx->lu;
   dev_free(ctx, L.ipiv);
   dev_free(ctx, L.perm);
+  dev_free(ctx, L.panel_u);
   dev_free(ctx, L.slot_val);
   dev_free(ctx, L.slot_row);
   dev_free(ctx, L.cand);

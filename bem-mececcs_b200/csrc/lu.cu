@@ -38,6 +38,9 @@
 
 #include <algorithm>
 #include <climits>
+#include <map>
+#include <mutex>
+#include <type_traits>
 
 #include "bem_internal.h"
 
@@ -155,6 +158,8 @@ struct PanelArgs {
   int pidx;
   int async_mail;  // k_panel_push: mailboxes filled by st.async (mbarrier complete_tx), no per-column cluster barrier
   int no_singular;  // a tournament round of a tall panel: a zero pivot is not an error here
+  int sl, rps;      // k_panel_ip: columns of a slice, row pitch of its shared-memory copy
+  void* ubuf;       // k_panel_ip: [B][64][64] U of the panel, while it runs
   // grid fallback only:
   void* slot_val;
   int* slot_row;
@@ -2801,6 +2806,7 @@ struct TrsvArgs {
   const void* A;
   size_t lda, bstride;
   int nn, batch, group, npanels, forward;
+  int b0;             // first problem of this launch (k_trsv_f32)
   const int* pstart;  // [npanels + 1] first row of each forward panel, then nn
   const int* perm;    // [panel][batch][kPermStride] gather lists
   void* v;            // problem b at v + b * vstride: right-hand side in, solution out
@@ -3096,7 +3102,7 @@ __global__ void __launch_bounds__(256) k_trsv_f32(const __grid_constant__ CUtens
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ int s_pl[kPermStride];  // the step's gather list: count, then dst/src pairs
   __shared__ int s_ok;
-  const int prob = blockIdx.x / a.group, rank = blockIdx.x % a.group, G = a.group;
+  const int prob = a.b0 + blockIdx.x / a.group, rank = blockIdx.x % a.group, G = a.group;
   if (prob >= a.batch) return;
   const unsigned long long wlim = wait_limit(a.status);
   float2* v = static_cast<float2*>(a.v) + (size_t)prob * a.vstride;
@@ -3327,6 +3333,8 @@ __global__ void __launch_bounds__(256) k_trsv_f32(const __grid_constant__ CUtens
   for (int r = lo + tid; r < hi; r += blockDim.x) v[r] = __ldcg(&xo[r]);
 }
 
+#include "panel.cuh"
+
 // ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
@@ -3343,6 +3351,9 @@ int lu_ensure_workspace(bem_ctx* ctx, int nn, int batch) {
   dev_free(ctx, L.pstart);
   L.pstart = nullptr;
   BEM_CUDA(ctx, dev_alloc(ctx, &L.pstart, (size_t)(max_panels + 1) * sizeof(int)));
+  dev_free(ctx, L.panel_u);
+  L.panel_u = nullptr;
+  BEM_CUDA(ctx, dev_alloc(ctx, &L.panel_u, (size_t)batch * 64 * 64 * sizeof(double2)));
   L.cap_nn = nn;
   L.cap_batch = batch;
   if (!L.slot_val) {
@@ -3524,6 +3535,147 @@ static int cluster_size_for(bem_ctx* ctx, int nn) {
   return cs;
 }
 
+// ---- k_panel_ip: shapes and launch ----
+struct PanelShape {
+  int cs = 0;        // CTAs per problem (0: too tall for this kernel)
+  int rp = 0, rps = 0, sl = 0;
+};
+
+// Largest number of panel rows a CTA's threads hold (RW = 8 row warps).
+template <typename R>
+constexpr int kPanelIpRows = sizeof(R) == 4 ? 8 * 32 * 8 : 8 * 32 * 2;
+
+static int panel_even(int rows) { return (rows + 1) & ~1; }  // even: 16-byte column starts of complex64
+// Pitch = 2 mod 16: conflict-free fragments of 4 columns x 4 rows.
+static int panel_pitch(int rp) { return (rp - 2 + 15) / 16 * 16 + 2; }
+
+// Columns of a slice (a multiple of 8, at most 64) for rp rows per CTA; 0 if
+// not even 8 fit.
+template <typename R>
+static int panel_slice(int rp) {
+  constexpr size_t kStatic = sizeof(R) == 4 ? 11 * 1024 : 19 * 1024;  // the kernel's static shared memory, rounded up
+  for (int sl = 64; sl >= 8; sl -= 8)
+    if (PanelIp<R>::smem(sl, panel_pitch(rp), 64) + kStatic + 1024 <= (size_t)227 * 1024) return sl;
+  return 0;
+}
+
+// Fewest CTAs a panel of m rows is given, which also fixes its slices (so the
+// factors do not depend on how many problems run together).  FP32: up to 416
+// rows per CTA, one 64-column slice, while 8 CTAs do (n <= 3328: 102 us for a
+// panel of 2871 rows against 140 in slices of 32 on 4 CTAs); then 8 CTAs up to
+// 832 rows each (slices of 32: 148 us at 6480 rows, but 16 problems at a time,
+// where 16-CTA clusters take 117 us for 7), then 16.  FP64: up to 200 rows
+// (one slice) while 8 CTAs do, then up to 256, then 16 CTAs.
+template <typename R>
+static int panel_cs_min(int m, int cs_max) {
+  int cs = 1;
+  if (sizeof(R) == 4) {
+    while (cs < 8 && m > 416 * cs) cs *= 2;
+    if (m > 832 * 8) cs = 16;
+  } else {
+    while (cs < 8 && m > 200 * cs) cs *= 2;
+    if (m > 256 * 8) cs = 16;
+  }
+  return std::min(cs, cs_max);
+}
+
+// Clusters of cs panel CTAs (one per SM) the device keeps resident at once.
+static int panel_resident(bem_ctx* ctx, int cs);
+
+// The panel of m rows of `batch` problems: more CTAs per problem than the
+// fewest while all problems' clusters stay resident together and the rows per
+// CTA are above about 230 (FP32) or 100 (FP64), below which a step no longer
+// gets faster (720 rows: 82 us on 8 CTAs, 86 on 4, 98 on 2).
+template <typename R>
+static PanelShape panel_shape(bem_ctx* ctx, int m, int batch) {
+  const int cs_max = cluster_size(ctx);
+  PanelShape s;
+  int cs = panel_cs_min<R>(m, cs_max);
+  s.sl = panel_slice<R>(panel_even((m + cs - 1) / cs));
+  if (s.sl == 0 || panel_even((m + cs - 1) / cs) > kPanelIpRows<R>) return s;
+  const int enough = sizeof(R) == 4 ? 230 : 100;
+  while (cs < cs_max && m > enough * cs && batch <= panel_resident(ctx, 2 * cs)) cs *= 2;
+  if (!ctx->small_clusters) cs = cs_max;
+  s.cs = cs;
+  s.rp = panel_even((m + cs - 1) / cs);
+  s.rps = panel_pitch(s.rp);
+  return s;
+}
+
+template <typename R, int RW, int RPT>
+static int launch_panel_ip_t(bem_ctx* ctx, const PanelArgs& pa, int batch) {
+  const size_t smem = PanelIp<R>::smem(pa.sl, pa.rps, pa.w);
+  auto kern = k_panel_ip<R, RW, RPT>;
+  BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(kern), smem));
+  BEM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(pa.cs, batch, 1);
+  cfg.blockDim = dim3(RW * 32 + 128, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = pa.cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  BEM_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, pa));
+  return BEM_OK;
+}
+
+// Row warps and rows per thread: measured fastest at each count (eight row
+// warps once two rows per thread on four would be needed, except FP64 up to
+// 256 rows).
+template <typename R>
+static int launch_panel_ip(bem_ctx* ctx, const PanelArgs& pa, int batch) {
+  if (pa.rp <= 128) return launch_panel_ip_t<R, 4, 1>(ctx, pa, batch);
+  if constexpr (sizeof(R) == 8) {
+    if (pa.rp <= 256) return launch_panel_ip_t<R, 4, 2>(ctx, pa, batch);
+    return launch_panel_ip_t<R, 8, 2>(ctx, pa, batch);
+  } else {
+    if (pa.rp <= 256) return launch_panel_ip_t<R, 8, 1>(ctx, pa, batch);
+    if (pa.rp <= 512) return launch_panel_ip_t<R, 8, 2>(ctx, pa, batch);
+    if (pa.rp <= 1024) return launch_panel_ip_t<R, 8, 4>(ctx, pa, batch);
+    return launch_panel_ip_t<R, 8, 8>(ctx, pa, batch);
+  }
+}
+
+static int panel_resident(bem_ctx* ctx, int cs) {
+  if (cs == 1) return ctx->num_sms;
+  // occupancy queries take tens of microseconds: one per device and cluster size
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  int& n = known[{ctx->device, cs}];
+  if (n) return n;
+  auto kern = k_panel_ip<float, 8, 4>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs, 1, 1);
+  cfg.blockDim = dim3(8 * 32 + 128, 1, 1);
+  cfg.dynamicSmemBytes = PanelIp<float>::smem(32, panel_pitch(800), 64);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int q = 0;
+  if (raise_smem_limit(reinterpret_cast<const void*>(kern), cfg.dynamicSmemBytes) != cudaSuccess ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&q, kern, &cfg) != cudaSuccess || q < 1)
+    q = std::max(1, ctx->num_sms / (2 * cs));
+  cudaGetLastError();
+  n = std::min(q, std::max(1, ctx->num_sms / cs));
+  return n;
+}
+
+// Is the default panel kernel in use (mailboxes filled by st.async)?
+static bool panel_ip_on(const bem_ctx* ctx, bool fp32) {
+  return ctx->panel_push && ctx->panel_async && !(fp32 && ctx->panel_calu);
+}
+
 // Clusters of the panel kernel that can be resident at once (0 if unknown).
 template <typename R, int NB, int NT>
 static int cluster_capacity(int cs, int rp) {
@@ -3551,6 +3703,10 @@ static int cluster_capacity(int cs, int rp) {
 
 template <typename R>
 static int lockstep_capacity_t(bem_ctx* ctx, int nn) {
+  if (panel_ip_on(ctx, sizeof(R) == 4)) {
+    const PanelShape ps = panel_shape<R>(ctx, nn, kMaxBatch + ctx->num_sms);  // the fewest CTAs per problem
+    if (ps.cs) return std::min(panel_resident(ctx, ps.cs), kMaxBatch);
+  }
   const int cs = cluster_size_for(ctx, nn);
   const int rp = (nn + cs - 1) / cs;
   if (rp > 512) return kMaxBatch;  // grid-panel fallback: problems take turns anyway
@@ -3651,7 +3807,7 @@ void release_cublas(bem_ctx* ctx) {
 // kernel, as many clusters as can be resident at once.
 int lu_lockstep_capacity(bem_ctx* ctx, int nn, bool fp32) {
   // occupancy queries are host calls of tens of microseconds: remember each answer
-  const long long key = 4LL * nn + (fp32 ? 1 : 0) + (ctx->small_clusters ? 2 : 0);
+  const long long key = 8LL * nn + (fp32 ? 1 : 0) + (ctx->small_clusters ? 2 : 0) + (panel_ip_on(ctx, fp32) ? 4 : 0);
   auto it = ctx->lockstep_cache.find(key);
   if (it != ctx->lockstep_cache.end()) return it->second;
   const int cap = fp32 ? lockstep_capacity_t<float>(ctx, nn) : lockstep_capacity_t<double>(ctx, nn);
@@ -3769,24 +3925,29 @@ static int trsv_f32(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, int
   LuWork& L = ctx->lu;
   done = false;
   const int npan = (int)L.panels.size(), nblk = (nn + kTrsvBlk - 1) / kTrsvBlk;
-  // the largest group (at most 64 CTAs per problem) whose CTAs are all resident
-  int group = 0, ldl = 0;
+  // The largest group (at most 64 CTAs per problem) whose CTAs are all
+  // resident; a share is at most 256 rows (one TMA box), so a large batch of
+  // large systems is solved by several launches of fewer problems.
+  int group = 0, ldl = 0, sub = batch;
   size_t smem = 0;
-  for (int g = std::min(64, std::max(1, nblk)); g >= 1; --g) {
-    const int per = (nn + g - 1) / g;
-    const int l = (per + 3) & ~1;  // rows of a share rounded out to even ends
-    const size_t sm = (size_t)kTrsvBlk * l * sizeof(float2) + (size_t)l * sizeof(int) + 128;
-    if (sm > kTrsvF32SmemMax || l > 256) break;  // smaller groups only need more; TMA boxes <= 256 rows
-    BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_trsv_f32), sm));
-    int occ = 0;
-    BEM_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trsv_f32, 256, sm));
-    int slots = occ * ctx->num_sms;
-    if (ctx->trsv_ctas > 0) slots = std::min(slots, ctx->trsv_ctas);
-    if (g * batch <= slots) {
-      group = g;
-      ldl = l;
-      smem = sm;
-      break;
+  for (int parts = 1; !group && parts <= batch; ++parts) {
+    sub = (batch + parts - 1) / parts;
+    for (int g = std::min(64, std::max(1, nblk)); g >= 1; --g) {
+      const int per = (nn + g - 1) / g;
+      const int l = (per + 3) & ~1;  // rows of a share rounded out to even ends
+      const size_t sm = (size_t)kTrsvBlk * l * sizeof(float2) + (size_t)l * sizeof(int) + 128;
+      if (sm > kTrsvF32SmemMax || l > 256) break;  // smaller groups only need more; TMA boxes <= 256 rows
+      BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_trsv_f32), sm));
+      int occ = 0;
+      BEM_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trsv_f32, 256, sm));
+      int slots = occ * ctx->num_sms;
+      if (ctx->trsv_ctas > 0) slots = std::min(slots, ctx->trsv_ctas);
+      if (g * sub <= slots) {
+        group = g;
+        ldl = l;
+        smem = sm;
+        break;
+      }
     }
   }
   if (!group) return BEM_OK;
@@ -3829,10 +3990,12 @@ static int trsv_f32(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, int
   CUtensorMap tm;
   if (!make_rows_map(&tm, A, nn, lda, bstride, batch, ldl)) return BEM_OK;  // k_trsv instead
   BEM_CUDA(ctx, cudaMemsetAsync(L.trsv_ctr, 0, batch * sizeof(unsigned), ctx->stream));
-  void* args[] = {&tm, &t, &tinv, &ldl, const_cast<int*>(&npan)};
-  BEM_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k_trsv_f32, dim3(group * batch), dim3(256), args, smem,
-                                            ctx->stream));
-  ctx->launches++;
+  for (t.b0 = 0; t.b0 < batch; t.b0 += sub) {
+    void* args[] = {&tm, &t, &tinv, &ldl, const_cast<int*>(&npan)};
+    BEM_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k_trsv_f32, dim3(group * std::min(sub, batch - t.b0)),
+                                              dim3(256), args, smem, ctx->stream));
+    ctx->launches++;
+  }
   done = true;
   return BEM_OK;
 }
@@ -3917,7 +4080,9 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
   // panel needs the cooperative-grid kernel.
   // FP32 (the mixed form) pivots by tournament per 8-column sub-panel.
   const bool calu = sizeof(R) == 4 && ctx->panel_calu;
+  const bool ip = panel_ip_on(ctx, sizeof(R) == 4);
   auto panel_nb = [&](int m) {
+    if (ip && panel_shape<R>(ctx, m, batch).cs) return 64;
     const int rp_c = (m + cs - 1) / cs;
     if (rp_c <= 512)
       for (int cand : {64, 32, 16})
@@ -3944,7 +4109,19 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     pa.async_mail = ctx->panel_async ? 1 : 0;
     const int nb = panel_nb(m);
     ProfScope ps(ctx, 1, 0.0, 2.0 * (double)m * std::min(nb ? nb : 64, m) * es * batch);
-    if (nb) {
+    const PanelShape sh = ip ? panel_shape<R>(ctx, m, batch) : PanelShape{};
+    if (sh.cs) {
+      w = std::min(64, m);
+      pa.w = w;
+      pa.cs = sh.cs;
+      pa.rp = sh.rp;
+      pa.rps = sh.rps;
+      pa.sl = sh.sl;
+      pa.ubuf = L.panel_u;
+      int rc = launch_panel_ip<R>(ctx, pa, batch);
+      if (rc) return rc;
+      ctx->launches++;
+    } else if (nb) {
       w = std::min(nb, m);
       pa.w = w;
       pa.rp = (m + cs - 1) / cs;

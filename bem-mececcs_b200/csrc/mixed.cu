@@ -133,10 +133,11 @@ void free_sweep(bem_ctx* ctx, SweepBuf& S) {
   S = SweepBuf{};
 }
 
+int alloc_sweep(bem_ctx* ctx, int batch, bool mixed, bool keep_g);
+
 int ensure_sweep(bem_ctx* ctx, int batch, bool mixed, bool keep_g = false) {
   SweepBuf& S = ctx->sweep;
   const int nn = 3 * ctx->mesh.nbe;
-  const int nbe = ctx->mesh.nbe;
   const int chunks = rhs_chunks(ctx);
   if (S.nn == nn && S.batch >= batch && (!mixed || S.A32) && (!keep_g || S.G64) && S.rhs_chunks >= chunks)
     return BEM_OK;
@@ -144,6 +145,19 @@ int ensure_sweep(bem_ctx* ctx, int batch, bool mixed, bool keep_g = false) {
   BEM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   release_sweep_graph(ctx);
   free_sweep(ctx, S);
+  const int rc = alloc_sweep(ctx, batch, mixed, keep_g);
+  if (rc) {  // no half-made buffers, no pending error: the caller may retry with fewer problems
+    free_sweep(ctx, S);
+    cudaGetLastError();
+  }
+  return rc;
+}
+
+int alloc_sweep(bem_ctx* ctx, int batch, bool mixed, bool keep_g) {
+  SweepBuf& S = ctx->sweep;
+  const int nn = 3 * ctx->mesh.nbe;
+  const int nbe = ctx->mesh.nbe;
+  const int chunks = rhs_chunks(ctx);
   S.nn = nn;
   S.batch = batch;
   S.lda = (size_t)((nn + 1) & ~1);  // even: 16-byte aligned column strides for the FP32 TMA maps
@@ -218,7 +232,18 @@ int sweep(bem_ctx* ctx, const double zge[2], const double zcs[2], const double z
     return fail(ctx, BEM_ERR_ARG, "bem_sweep: batch, count or refinement steps out of range");
   // No more problems in lockstep than the panel kernel keeps resident at once.
   batch = std::min(batch, lu_lockstep_capacity(ctx, 3 * ctx->mesh.nbe, mixed));
+  // As few steps as the limit allows, of even size (28 frequencies at a limit
+  // of 18 run as 14 + 14), and no larger than there is memory for.
+  auto even = [&](int limit) {
+    const int steps = (std::max(nfreq, 1) + limit - 1) / limit;
+    return (std::max(nfreq, 1) + steps - 1) / steps;
+  };
+  batch = even(batch);
   int rc = ensure_sweep(ctx, batch, mixed);
+  while (rc == BEM_ERR_NOMEM && batch > 1) {
+    batch = even((batch + 1) / 2);
+    rc = ensure_sweep(ctx, batch, mixed);
+  }
   if (rc) return rc;
   SweepBuf& S = ctx->sweep;
   const int nn = S.nn;

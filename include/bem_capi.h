@@ -306,8 +306,10 @@ int bem_batch_solve(bem_ctx *driver, int nprob, bem_ctx *const *probs,
                     double *const *x_out, double *corr_out);
 
 /* Largest lockstep batch bem_sweep uses for this mesh and form: the number
- * of panel-factorisation thread-block clusters the device keeps resident at
- * once (7 for n = 6480 on a 148-SM B200), capped at 64. */
+ * of panel-factorisation thread-block clusters (of the fewest CTAs the size
+ * allows) the device keeps resident at once, capped at 64.  A sweep runs in
+ * as few steps as this allows, of even size, and in smaller ones when their
+ * systems do not fit the device's memory. */
 int bem_sweep_batch_limit(bem_ctx *ctx, int form, int *limit);
 
 /* Kernel-class timing with CUDA events on ctx's stream.  Classes:

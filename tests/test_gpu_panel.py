@@ -1,0 +1,59 @@
+"""The LU panel kernel (csrc/panel.cuh) at the edges of its row tiles, slices
+and clusters, through the public solves, against numpy and the plain form."""
+import numpy as np
+import pytest
+
+from bem_mececcs_b200 import capi, meshgen
+from bem_mececcs_b200.solver import BemSolver, solve_dense
+from gpu_util import rel
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(kind, n, rng):
+    if kind == "random":
+        return rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    if kind == "dominant":  # pivots stay on the diagonal
+        return 0.5 * np.eye(n) + 0.01 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n)
+    # every candidate of the first column has the same |re| + |im|
+    a = (1j ** rng.integers(0, 4, (n, n))) * 0.5 + 0.1 * rng.standard_normal((n, n))
+    a[:, 0] = 1j ** rng.integers(0, 4, n)
+    return a
+
+
+# one row, a sub-panel, a panel and one more, one slice of 64 (up to 200 rows a
+# CTA), slices of 56 and fewer columns, clusters of 1 to 16 CTAs
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 64, 65, 201, 400, 1633, 2049])
+@pytest.mark.parametrize("kind", ["random", "dominant", "ties"])
+@pytest.mark.parametrize("clusters", [True, False], ids=["sized", "16"])
+def test_fp64_panel(n, kind, clusters):
+    """Backward error of the solve: LU with partial pivoting stays below
+    n eps times the element growth, which for these matrices is far below 10."""
+    rng = np.random.default_rng(n)
+    a = _matrix(kind, n, rng)
+    b = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    ctx = capi.Context(0)
+    ctx.set_option("small_clusters", clusters)
+    x = solve_dense(ctx, a, b)
+    ctx.close()
+    err = np.linalg.norm(a @ x - b) / (np.linalg.norm(a, 2 if n < 500 else "fro") * np.linalg.norm(x) + np.linalg.norm(b))
+    assert err < 10 * max(n, 8) * np.finfo(float).eps
+
+
+# n = 12..234: clusters of 1 to 2 CTAs and ragged last panels; 3366: slices of
+# 32 columns on 8 CTAs until 3328 rows are left
+@pytest.mark.parametrize("nx,ny", [(2, 2), (23, 1), (8, 8), (13, 6), (34, 33)])
+def test_fp32_panel(nx, ny):
+    """The mixed form reaches the plain form's solution (1e-10) whether its
+    problems run alone or together."""
+    m = meshgen.enclosed_grid(nx, ny, jitter=0.10, seed=3, depth=2.5, layers=2)
+    d = meshgen.traction_patch(m, radius=6.0)
+    with BemSolver(m) as sol:
+        sol.ghmatece()
+        sol.set_bc(d.kode, d.bc, d.dam, d.rho)
+        freqs = [0.4, 1.1, 2.7]
+        xp, _ = sol.sweep(freqs, form="plain", batch=3)
+        for batch in (1, 3):
+            xm, _ = sol.sweep(freqs, form="mixed", batch=batch, refine=4)
+            for i in range(len(freqs)):
+                assert rel(xm[i], xp[i]) < 1e-10, (batch, freqs[i])
