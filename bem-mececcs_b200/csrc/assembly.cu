@@ -21,6 +21,11 @@
 
 namespace bem {
 
+// Packed index of a symmetric 3x3 entry: 00 01 02 11 12 22.
+__host__ __device__ constexpr int sym3(int i, int j) {
+  return i <= j ? (i == 0 ? j : (i == 1 ? 2 + j : 5)) : (j == 0 ? i : (j == 1 ? 2 + i : 5));
+}
+
 struct GaussRule {
   double gi[kMaxNpg], ome[kMaxNpg];
   int npg;
@@ -124,6 +129,11 @@ __global__ void __launch_bounds__(128) k_static_rows(StaticParams p) {
   const int I = blockIdx.x * 32 + lane;
   const int J0 = blockIdx.y * p.jc;
   const int jn = min(p.jc, p.n - J0);
+  // the chunk's Gauss points in shared memory (read through the L1 cache, their
+  // latency was half of the warps' stalls)
+  extern __shared__ __align__(128) double4 s_sq[];
+  for (int i = threadIdx.x; i < jn * p.ng; i += blockDim.x) s_sq[i] = p.gq[(size_t)J0 * p.ng + i];
+  __syncthreads();
   double h[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) h[k] = 0.0;
@@ -133,29 +143,35 @@ __global__ void __launch_bounds__(128) k_static_rows(StaticParams p) {
       const int J = J0 + jl;
       if (J == I) continue;  // HEST(JJ:JJ+2,JJ:JJ+2) = 0 (Ghmatece.for:134-135)
       const double4 nv = p.eta[J];
-      const double4* q = p.gq + (size_t)J * p.ng;
-      double a0 = 0, b00 = 0, b01 = 0, b02 = 0, b11 = 0, b12 = 0, b22 = 0, c0 = 0, c1 = 0, c2 = 0;
+      const double4* q = s_sq + jl * p.ng;
+      // T_ij = C3/r^2 (...) with rd = r/|r|: per point the sums of
+      // u r_k, u = w / r^3, and of (3 w dr/dn / r^2) rd_i rd_j
+      // = (3 u (r.n) / r^2) r_i r_j; 32 FP64 operations, the constants and
+      // a0 = n . c applied once per element.
+      double b00 = 0, b01 = 0, b02 = 0, b11 = 0, b12 = 0, b22 = 0, c0 = 0, c1 = 0, c2 = 0;
+#pragma unroll 4
       for (int g = 0; g < p.ng; ++g) {
         const double4 qq = q[g];
-        double r1 = qq.x - P.x, r2 = qq.y - P.y, r3 = qq.z - P.z;
-        double r = sqrt(r1 * r1 + r2 * r2 + r3 * r3);
-        double ir = 1.0 / r;
-        double d0 = r1 * ir, d1 = r2 * ir, d2 = r3 * ir;
-        double drn = (r1 * nv.x + r2 * nv.y + r3 * nv.z) * ir;
-        double s = qq.w * p.c3 * ir * ir;
-        double sd = 3.0 * s * drn;
-        a0 = fma(s * p.c4, drn, a0);
-        b00 = fma(sd * d0, d0, b00);
-        b01 = fma(sd * d0, d1, b01);
-        b02 = fma(sd * d0, d2, b02);
-        b11 = fma(sd * d1, d1, b11);
-        b12 = fma(sd * d1, d2, b12);
-        b22 = fma(sd * d2, d2, b22);
-        double sc = s * p.c4;
-        c0 = fma(sc, d0, c0);
-        c1 = fma(sc, d1, c1);
-        c2 = fma(sc, d2, c2);
+        const double r1 = qq.x - P.x, r2 = qq.y - P.y, r3 = qq.z - P.z;
+        const double ir = rsqrt_fast(fma(r1, r1, fma(r2, r2, r3 * r3)));
+        const double ir2 = ir * ir;
+        const double u = (qq.w * ir) * ir2;
+        const double gs = (u * ir2) * fma(r1, nv.x, fma(r2, nv.y, r3 * nv.z));
+        const double g0 = gs * r1, g1 = gs * r2, g2 = gs * r3;
+        b00 = fma(g0, r1, b00);
+        b01 = fma(g0, r2, b01);
+        b02 = fma(g0, r3, b02);
+        b11 = fma(g1, r2, b11);
+        b12 = fma(g1, r3, b12);
+        b22 = fma(g2, r3, b22);
+        c0 = fma(u, r1, c0);
+        c1 = fma(u, r2, c1);
+        c2 = fma(u, r3, c2);
       }
+      const double s3 = 3.0 * p.c3, s4 = p.c3 * p.c4;
+      b00 *= s3, b01 *= s3, b02 *= s3, b11 *= s3, b12 *= s3, b22 *= s3;
+      c0 *= s4, c1 *= s4, c2 *= s4;
+      const double a0 = fma(c0, nv.x, fma(c1, nv.y, c2 * nv.z));
       const double nn_[3] = {nv.x, nv.y, nv.z};
       const double cc[3] = {c0, c1, c2};
       const double bb[3][3] = {{b00, b01, b02}, {b01, b11, b12}, {b02, b12, b22}};
@@ -195,54 +211,53 @@ __global__ void k_static_reduce(int nbe, int chunks, const double* __restrict__ 
 // GEST_SINGULAR on the device (src/Ghmatece.for:288-323, src/Singge.for:11-202):
 // per element, 4 triangles with corners 3 and 4 collapsed to the centroid,
 // each integrated with NPG x NPG points of the Kelvin U kernel
-// U_ij = C1/r (C2 d_ij + rd_i rd_j).
-__global__ void k_gest(int nbe, const double* __restrict__ corner, const double4* __restrict__ colloc,
-                       GaussRule rule, double c1, double c2, double* gestdiag, int* status) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nbe) return;
+// U_ij = C1/r (C2 d_ij + rd_i rd_j).  One thread per triangle, summed over
+// the element's 4 lanes (one thread per element left 17 CTAs of a 2160-element
+// mesh with a chain of 64 points each: 46 us).
+__global__ void __launch_bounds__(128) k_gest(int nbe, const double* __restrict__ corner,
+                                              const double4* __restrict__ colloc, GaussRule rule, double c1,
+                                              double c2, double* gestdiag, int* status) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = min(t >> 2, nbe - 1), it = t & 3;
   const double4 P = colloc[j];
-  double el[4][3];
+  double co[4][3];
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) el[k][c] = corner[(size_t)j * 12 + 3 * k + c];
-  double gsum[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) gsum[k] = 0.0;
-  for (int it = 0; it < 4; ++it) {
-    double co[4][3];
-    const int a = it, b = (it + 1) & 3;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      co[0][c] = el[a][c];
-      co[1][c] = el[b][c];
-    }
-    co[2][0] = co[3][0] = P.x;
-    co[2][1] = co[3][1] = P.y;
-    co[2][2] = co[3][2] = P.z;
-    double gp[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) gp[k] = 0.0;
-    for (int jg = 0; jg < rule.npg; ++jg)
-      for (int ig = 0; ig < rule.npg; ++ig) {
-        double x, y, z, det;
-        gauss_point(co, rule.gi[ig], rule.gi[jg], x, y, z, det);
-        if (det < 1.0e-5) atomicOr(&status[ST_DEGENERATE], 1);
-        double p12 = rule.ome[ig] * rule.ome[jg] * det;
-        double r1 = x - P.x, r2 = y - P.y, r3 = z - P.z;
-        double r = sqrt(r1 * r1 + r2 * r2 + r3 * r3);
-        double rd[3] = {r1 / r, r2 / r, r3 / r};
-#pragma unroll
-        for (int jj = 0; jj < 3; ++jj)
-#pragma unroll
-          for (int ii = 0; ii < 3; ++ii)
-            gp[3 * jj + ii] += ((c1 / r) * (c2 * (ii == jj ? 1.0 : 0.0) + rd[ii] * rd[jj])) * p12;
-      }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) gsum[k] = gsum[k] + gp[k];
+  for (int c = 0; c < 3; ++c) {
+    co[0][c] = corner[(size_t)j * 12 + 3 * it + c];
+    co[1][c] = corner[(size_t)j * 12 + 3 * ((it + 1) & 3) + c];
   }
+  co[2][0] = co[3][0] = P.x;
+  co[2][1] = co[3][1] = P.y;
+  co[2][2] = co[3][2] = P.z;
+  double iso = 0.0, gp[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // sums of w/r and of (w/r) rd_i rd_j
+  for (int jg = 0; jg < rule.npg; ++jg)
+    for (int ig = 0; ig < rule.npg; ++ig) {
+      double x, y, z, det;
+      gauss_point(co, rule.gi[ig], rule.gi[jg], x, y, z, det);
+      if (det < 1.0e-5) atomicOr(&status[ST_DEGENERATE], 1);
+      const double r1 = x - P.x, r2 = y - P.y, r3 = z - P.z;
+      const double ir = rsqrt_fast(fma(r1, r1, fma(r2, r2, r3 * r3)));
+      const double u = rule.ome[ig] * rule.ome[jg] * det * ir, v = u * (ir * ir);
+      const double v1 = v * r1, v2 = v * r2;
+      iso += u;
+      gp[0] = fma(v1, r1, gp[0]);
+      gp[1] = fma(v1, r2, gp[1]);
+      gp[2] = fma(v1, r3, gp[2]);
+      gp[3] = fma(v2, r2, gp[3]);
+      gp[4] = fma(v2, r3, gp[4]);
+      gp[5] = fma(v * r3, r3, gp[5]);
+    }
 #pragma unroll
-  for (int k = 0; k < 9; ++k) gestdiag[(size_t)j * 9 + k] = gsum[k];
+  for (int off = 1; off < 4; off <<= 1) {
+    iso += __shfl_xor_sync(0xffffffffu, iso, off);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) gp[k] += __shfl_xor_sync(0xffffffffu, gp[k], off);
+  }
+  if (it != 0 || (t >> 2) >= nbe) return;
+#pragma unroll
+  for (int jj = 0; jj < 3; ++jj)
+#pragma unroll
+    for (int ii = 0; ii < 3; ++ii)
+      gestdiag[(size_t)j * 9 + 3 * jj + ii] = c1 * ((ii == jj ? c2 * iso : 0.0) + gp[sym3(ii, jj)]);
 }
 
 // ---------------------------------------------------------------------------
@@ -274,13 +289,13 @@ struct DynCore {
 };
 // One mesh, `batch` frequencies (bem_ghmatecd, bem_sweep).
 struct DynParams : DynCore {
-  StokesConsts<double> kb[kMaxBatch];  // per problem (frequency)
+  StokesConsts kb[kMaxBatch];  // per problem (frequency)
 };
 // One problem of a grouped launch (bem_batch_solve): its own mesh, BCs and
 // constants; its system is padded to npad unknowns, the right-hand side in
 // column npad.
 struct DynProblem : DynCore {
-  StokesConsts<double> kc;
+  StokesConsts kc;
   int npad;
 };
 
@@ -292,45 +307,61 @@ __device__ __forceinline__ void st(double2* p, zd z) { *p = make_double2(z.re, z
 
 // Diagonal blocks (I == J): SING_DE (src/Sing_de.for:13-113) with SOLFUNDIF
 // (src/Solfundif.for:18-69), Stokes minus Kelvin per Gauss point, plus the
-// static diagonals (src/Ghmatecd.for:150-153).  One thread per element.
-__device__ __forceinline__ void dyn_diag_body(const DynCore& p, const StokesConsts<double>& kc, int prob) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= p.nbe) return;
+// static diagonals (src/Ghmatecd.for:150-153).  kDiagLanes threads per element
+// share its Gauss points and sum by shuffles: with one thread per element the
+// kernel was one long chain of 16 to 64 evaluations on a few CTAs.
+constexpr int kDiagLanes = 8;
+
+__device__ __forceinline__ void dyn_diag_body(const DynCore& p, const StokesConsts& kc, int prob) {
+  __shared__ CexpTable tab;
+  cexp_table_fill(tab);
+  __syncthreads();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = min(t / kDiagLanes, p.nbe - 1), part = t % kDiagLanes;
   double2* diag_h = p.diag_h + (size_t)prob * p.nbe * 9;
   double2* diag_g = p.diag_g + (size_t)prob * p.nbe * 9;
   const double4 P = p.colloc[j];
   const double4 nv = p.eta[j];
-  const double rn0 = nv.x, rn1 = nv.y, rn2 = nv.z;
+  const double rn[3] = {nv.x, nv.y, nv.z};
   zd zh[9], zg[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) zh[k] = zg[k] = zd{0.0, 0.0};
   const double4* q = p.gq + (size_t)j * p.ng;
-  for (int g = 0; g < p.ng; ++g) {
+  for (int g = part; g < p.ng; g += kDiagLanes) {
     const double4 qq = q[g];
     double r1 = qq.x - P.x, r2 = qq.y - P.y, r3 = qq.z - P.z;
-    const double ir = rsqrt(fma(r1, r1, fma(r2, r2, r3 * r3)));  // r and 1/r from one rsqrt
-    const double r = fma(r1, r1, fma(r2, r2, r3 * r3)) * ir;
-    double drn = (r1 * rn0 + r2 * rn1 + r3 * rn2) * ir;
+    const double rr = fma(r1, r1, fma(r2, r2, r3 * r3));
+    const double ir = rsqrt_fast(rr);  // r and 1/r from one reciprocal square root
+    const double r = rr * ir;
+    double drn = (r1 * rn[0] + r2 * rn[1] + r3 * rn[2]) * ir;
     const double rd[3] = {r1 * ir, r2 * ir, r3 * ir};
-    const double rn[3] = {rn0, rn1, rn2};
-    StokesRadial<double> s = stokes_radial(kc, r, ir);
+    const StokesRadial s = stokes_radial(kc, tab, r, ir);
 #pragma unroll
     for (int jj = 0; jj < 3; ++jj)
 #pragma unroll
       for (int ii = 0; ii < 3; ++ii) {
         const double dl = (ii == jj) ? 1.0 : 0.0;
         zd u = kc.zc0 * (s.fhi * dl - s.cappa * (rd[jj] * rd[ii]));
-        zd t = kc.inv4pi * ((s.aa * (drn * dl + rd[jj] * rn[ii])) + s.bb * (rd[ii] * rd[jj] * drn) +
-                            s.cc * (rd[ii] * rn[jj]));
+        zd t2 = kc.inv4pi * ((s.aa * (drn * dl + rd[jj] * rn[ii])) + s.bbh * (2.0 * rd[ii] * rd[jj] * drn) +
+                             s.cc * (rd[ii] * rn[jj]));
         if (p.fast_singular) {
-          u.re -= (p.c1 / r) * (p.c2 * dl + rd[ii] * rd[jj]);
-          t.re -= (p.c3 * ir * ir) * (drn * (p.c4 * dl + 3.0 * rd[ii] * rd[jj]) +
-                                      p.c4 * (rd[jj] * rn[ii] - rd[ii] * rn[jj]));
+          u.re -= (p.c1 * ir) * (p.c2 * dl + rd[ii] * rd[jj]);
+          t2.re -= (p.c3 * ir * ir) * (drn * (p.c4 * dl + 3.0 * rd[ii] * rd[jj]) +
+                                       p.c4 * (rd[jj] * rn[ii] - rd[ii] * rn[jj]));
         }
-        cfma(zh[3 * jj + ii], t, qq.w);
+        cfma(zh[3 * jj + ii], t2, qq.w);
         cfma(zg[3 * jj + ii], u, qq.w);
       }
   }
+#pragma unroll
+  for (int k = 0; k < 9; ++k)
+#pragma unroll
+    for (int off = 1; off < kDiagLanes; off <<= 1) {
+      zh[k].re += __shfl_xor_sync(0xffffffffu, zh[k].re, off);
+      zh[k].im += __shfl_xor_sync(0xffffffffu, zh[k].im, off);
+      zg[k].re += __shfl_xor_sync(0xffffffffu, zg[k].re, off);
+      zg[k].im += __shfl_xor_sync(0xffffffffu, zg[k].im, off);
+    }
+  if (part != 0 || t / kDiagLanes >= p.nbe) return;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     if (p.fast_singular) {
@@ -347,7 +378,7 @@ __global__ void __launch_bounds__(128) k_dyn_diag(DynParams p) { dyn_diag_body(p
 // Grouped form: blockIdx.z is the problem; its descriptor is in global memory.
 __global__ void __launch_bounds__(128) k_dyn_diag_grp(const DynProblem* __restrict__ g) {
   const DynProblem& p = g[blockIdx.z];
-  const StokesConsts<double> kc = p.kc;
+  const StokesConsts kc = p.kc;
   dyn_diag_body(p, kc, 0);
 }
 
@@ -357,16 +388,13 @@ __global__ void __launch_bounds__(128) k_dyn_diag_grp(const DynProblem* __restri
 // not stored.  Diagonal pairs take their blocks from k_dyn_diag.
 constexpr int kRowsPerCta = 32;
 
-// Packed index of a symmetric 3x3 entry: 00 01 02 11 12 22.
-__host__ __device__ constexpr int sym3(int i, int j) {
-  return i <= j ? (i == 0 ? j : (i == 1 ? 2 + j : 5)) : (j == 0 ? i : (j == 1 ? 2 + i : 5));
-}
 constexpr int kWarpsPerCta = 4;
 
-__device__ __forceinline__ void dyn_offdiag_body(const DynCore& p, const StokesConsts<double>& kc, int prob) {
+__device__ __forceinline__ void dyn_offdiag_body(const DynCore& p, const StokesConsts& kc, int prob) {
   extern __shared__ __align__(128) double4 s_gq[];  // [jc][ng]
   __shared__ uint64_t s_bar;
   __shared__ zd s_rhs[kWarpsPerCta][3 * kRowsPerCta];
+  __shared__ CexpTable tab;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int I = blockIdx.x * kRowsPerCta + lane;
   const int J0 = blockIdx.y * p.jc;
@@ -381,6 +409,7 @@ __device__ __forceinline__ void dyn_offdiag_body(const DynCore& p, const StokesC
   const double2* diag_g = p.diag_g + (size_t)prob * p.nbe * 9;
   const bool preswap = p.zh_pre && prob == 0;
 
+  cexp_table_fill(tab);
   if (threadIdx.x == 0) mbar_init(&s_bar, 1);
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -405,48 +434,54 @@ __device__ __forceinline__ void dyn_offdiag_body(const DynCore& p, const StokesC
     const double n3[3] = {nv.x, nv.y, nv.z};
     zd U[3][3], T[3][3];  // [i][j]: row component i, column component j
     if (valid && J != I) {
-      zd F{0, 0}, A0{0, 0};
+      zd F{0, 0};
       zd K[6], B[6], A1[3], C[3];
 #pragma unroll
       for (int k = 0; k < 6; ++k) K[k] = B[k] = zd{0, 0};
 #pragma unroll
       for (int k = 0; k < 3; ++k) A1[k] = C[k] = zd{0, 0};
       const double4* q = s_gq + jl * p.ng;
-#pragma unroll 2
+      // About 190 FP64 operations per point (275 with the general exp, sincos
+      // and rsqrt and the radial functions term by term).
+#pragma unroll 1
       for (int g = 0; g < p.ng; ++g) {
         const double4 qq = q[g];
         const double r1 = qq.x - P.x, r2 = qq.y - P.y, r3 = qq.z - P.z;
         const double rr = fma(r1, r1, fma(r2, r2, r3 * r3));
-        const double ir = rsqrt(rr);  // r and 1/r from one rsqrt
+        const double ir = rsqrt_fast(rr);  // r and 1/r from one reciprocal square root
         const double r = rr * ir;
         const double d0 = r1 * ir, d1 = r2 * ir, d2 = r3 * ir;
-        const double drn = (r1 * n3[0] + r2 * n3[1] + r3 * n3[2]) * ir;
-        const StokesRadial<double> s = stokes_radial(kc, r, ir);
+        const double drn = d0 * n3[0] + d1 * n3[1] + d2 * n3[2];
+        const StokesRadial s = stokes_radial(kc, tab, r, ir);
         const double wt = qq.w;
-        const double w0 = wt * d0, w1 = wt * d1, w2 = wt * d2, wd = wt * drn;
+        const double w0 = wt * d0, w1 = wt * d1, w2 = wt * d2;
+        const double k0 = w0 * d0, k1 = w0 * d1, k2 = w0 * d2, k3 = w1 * d1, k4 = w1 * d2, k5 = w2 * d2;
         cfma(F, s.fhi, wt);
-        cfma(K[0], s.cappa, w0 * d0);
-        cfma(K[1], s.cappa, w0 * d1);
-        cfma(K[2], s.cappa, w0 * d2);
-        cfma(K[3], s.cappa, w1 * d1);
-        cfma(K[4], s.cappa, w1 * d2);
-        cfma(K[5], s.cappa, w2 * d2);
-        cfma(A0, s.aa, wd);
+        cfma(K[0], s.cappa, k0);
+        cfma(K[1], s.cappa, k1);
+        cfma(K[2], s.cappa, k2);
+        cfma(K[3], s.cappa, k3);
+        cfma(K[4], s.cappa, k4);
+        cfma(K[5], s.cappa, k5);
         cfma(A1[0], s.aa, w0);
         cfma(A1[1], s.aa, w1);
         cfma(A1[2], s.aa, w2);
-        const double e0 = wd * d0, e1 = wd * d1, e2 = wd * d2;
-        cfma(B[0], s.bb, e0 * d0);
-        cfma(B[1], s.bb, e0 * d1);
-        cfma(B[2], s.bb, e0 * d2);
-        cfma(B[3], s.bb, e1 * d1);
-        cfma(B[4], s.bb, e1 * d2);
-        cfma(B[5], s.bb, e2 * d2);
+        const zd bd = s.bbh * drn;
+        cfma(B[0], bd, k0);
+        cfma(B[1], bd, k1);
+        cfma(B[2], bd, k2);
+        cfma(B[3], bd, k3);
+        cfma(B[4], bd, k4);
+        cfma(B[5], bd, k5);
         cfma(C[0], s.cc, w0);
         cfma(C[1], s.cc, w1);
         cfma(C[2], s.cc, w2);
       }
-      // U_ij = c0 (d_ij F - K_ij); T_ij = (d_ij A0 + n_i A1_j + B_ij + n_j C_i) / 4pi.
+      // sum of AA dr/dn = n . A1, as dr/dn = n . r/|r| (one normal per element)
+      zd A0 = A1[0] * n3[0];
+      cfma(A0, A1[1], n3[1]);
+      cfma(A0, A1[2], n3[2]);
+      // U_ij = c0 (d_ij F - K_ij); T_ij = (d_ij A0 + n_i A1_j + 2 B_ij + n_j C_i) / 4pi (B sums BB / 2).
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -454,7 +489,7 @@ __device__ __forceinline__ void dyn_offdiag_body(const DynCore& p, const StokesC
           const int sy = sym3(i, j);
           zd u = (i == j) ? F - K[sy] : -K[sy];
           U[i][j] = kc.zc0 * u;
-          zd t = B[sy];
+          zd t = B[sy] * 2.0;
           cfma(t, A1[j], n3[i]);
           cfma(t, C[i], n3[j]);
           if (i == j) t = t + A0;
@@ -511,11 +546,11 @@ __device__ __forceinline__ void dyn_offdiag_body(const DynCore& p, const StokesC
   }
 }
 
-__global__ void __launch_bounds__(128) k_dyn_offdiag(DynParams p) {
+__global__ void __launch_bounds__(128, 3) k_dyn_offdiag(DynParams p) {
   dyn_offdiag_body(p, p.kb[blockIdx.z], blockIdx.z);
 }
 
-__global__ void __launch_bounds__(128) k_dyn_offdiag_grp(const DynProblem* __restrict__ g) {
+__global__ void __launch_bounds__(128, 3) k_dyn_offdiag_grp(const DynProblem* __restrict__ g) {
   const DynProblem& p = g[blockIdx.z];
   dyn_offdiag_body(p, p.kc, 0);
 }
@@ -625,7 +660,7 @@ int launch_static(bem_ctx* ctx, const double c[4], int compute_gest, double* hes
   p.part = ctx->static_part;
   p.hest_full = hest_full;
   dim3 grid((m.nbe + kRowsPerCta - 1) / kRowsPerCta, chunks);
-  k_static_rows<<<grid, 128, 0, ctx->stream>>>(p);
+  k_static_rows<<<grid, 128, (size_t)jc * m.ng * sizeof(double4), ctx->stream>>>(p);
   ctx->launches++;
   BEM_CUDA(ctx, cudaGetLastError());
   k_static_reduce<<<(m.nbe * 9 + 255) / 256, 256, 0, ctx->stream>>>(m.nbe, chunks, ctx->static_part,
@@ -639,7 +674,7 @@ int launch_static(bem_ctx* ctx, const double c[4], int compute_gest, double* hes
       rule.gi[i] = m.gi[i];
       rule.ome[i] = m.ome[i];
     }
-    k_gest<<<(m.nbe + 127) / 128, 128, 0, ctx->stream>>>(m.nbe, m.corner, m.colloc, rule, c[0], c[1],
+    k_gest<<<(4 * m.nbe + 127) / 128, 128, 0, ctx->stream>>>(m.nbe, m.corner, m.colloc, rule, c[0], c[1],
                                                          ctx->gestdiag, ctx->d_status);
     ctx->launches++;
     BEM_CUDA(ctx, cudaGetLastError());
@@ -647,7 +682,7 @@ int launch_static(bem_ctx* ctx, const double c[4], int compute_gest, double* hes
   return BEM_OK;
 }
 
-StokesConsts<double> make_consts(const double zge_[2], const double zcs_[2],
+StokesConsts make_consts(const double zge_[2], const double zcs_[2],
                                         const double zcp_[2], double fr) {
   // Solfund.for:29-35 in double on the host.
   auto mul = [](double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); };
@@ -661,7 +696,7 @@ StokesConsts<double> make_consts(const double zge_[2], const double zcs_[2],
   double2 zcp = make_double2(zcp_[0], zcp_[1]);
   double2 zwi = make_double2(0.0, fr);
   double2 mzwi = make_double2(-zwi.x, -zwi.y);
-  StokesConsts<double> k{};
+  StokesConsts k{};
   double2 c0 = div(make_double2(1.0, 0.0), mul(make_double2(4.0 * pi, 0.0), zge));
   double2 pc = div(zcp, zcs), sc = div(zcs, zcp);
   double2 c1 = mul(pc, pc), c2 = mul(sc, sc);
@@ -675,6 +710,10 @@ StokesConsts<double> make_consts(const double zge_[2], const double zcs_[2],
   const double2 ikp = div(make_double2(1.0, 0.0), kp), iks = div(make_double2(1.0, 0.0), ks);
   k.izkp = zd{ikp.x, ikp.y};
   k.izks = zd{iks.x, iks.y};
+  const double2 ikp2 = mul(ikp, ikp), iks2 = mul(iks, iks);
+  k.izkp2 = zd{ikp2.x, ikp2.y};
+  k.izks2 = zd{iks2.x, iks2.y};
+  k.damped = kp.x != 0.0 || ks.x != 0.0;
   return k;
 }
 
@@ -769,7 +808,7 @@ int launch_dynamic_group(bem_ctx* wk, const GroupMember* mem, int count, void* h
   const DynProblem* dd = static_cast<const DynProblem*>(d_desc);
   BEM_CUDA(wk, cudaMemcpyAsync(d_desc, hd, (size_t)count * sizeof(DynProblem), cudaMemcpyHostToDevice, wk->stream));
   ProfScope ps(wk, 0, work, bytes);
-  k_dyn_diag_grp<<<dim3((max_nbe + 127) / 128, 1, count), 128, 0, wk->stream>>>(dd);
+  k_dyn_diag_grp<<<dim3((max_nbe * kDiagLanes + 127) / 128, 1, count), 128, 0, wk->stream>>>(dd);
   BEM_CUDA(wk, cudaGetLastError());
   k_dyn_offdiag_grp<<<dim3((max_nbe + kRowsPerCta - 1) / kRowsPerCta, max_chunks, count), 128, smem, wk->stream>>>(
       dd);
@@ -826,7 +865,7 @@ int launch_dynamic_batch(bem_ctx* ctx, const DynBatch& b) {
   // work: Stokes evaluations; bytes: the FP64 system (and its complex64 copy) written once
   ProfScope ps(ctx, 0, (double)m.nbe * (double)m.nbe * (double)m.ng * b.batch,
                (double)(3 * m.nbe) * (3 * m.nbe + 1) * (16.0 + (b.A32 ? 8.0 : 0.0)) * b.batch);
-  k_dyn_diag<<<dim3((m.nbe + 127) / 128, 1, b.batch), 128, 0, ctx->stream>>>(p);
+  k_dyn_diag<<<dim3((m.nbe * kDiagLanes + 127) / 128, 1, b.batch), 128, 0, ctx->stream>>>(p);
   ctx->launches++;
   BEM_CUDA(ctx, cudaGetLastError());
   const size_t smem = (size_t)jc * m.ng * sizeof(double4);
@@ -921,7 +960,7 @@ __global__ void __launch_bounds__(128) k_static_system(StaticSysParams p) {
         const double4 qq = q[g];
         const double r1 = qq.x - P.x, r2 = qq.y - P.y, r3 = qq.z - P.z;
         const double rr = fma(r1, r1, fma(r2, r2, r3 * r3));
-        const double ir = rsqrt(rr);
+        const double ir = rsqrt_fast(rr);
         const double rd[3] = {r1 * ir, r2 * ir, r3 * ir};
         const double rdn = rd[0] * n3[0] + rd[1] * n3[1] + rd[2] * n3[2];
         const double ct = p.c3 * ir * ir * qq.w, cu = p.c1 * ir * qq.w;
@@ -1124,7 +1163,7 @@ int bem_ghmatecd_noalloc(bem_ctx* ctx, const double zge[2], const double zcs[2],
   // timed as the assembly class when profiling is on, like bem_ghmatecd:
   // work = Stokes evaluations, bytes = the system written once
   ProfScope ps(ctx, 0, (double)m.nbe * (double)m.nbe * (double)m.ng, (double)nn * (nn + 1) * 16.0);
-  k_dyn_diag<<<dim3((m.nbe + 127) / 128, 1, 1), 128, 0, ctx->stream>>>(p);
+  k_dyn_diag<<<dim3((m.nbe * kDiagLanes + 127) / 128, 1, 1), 128, 0, ctx->stream>>>(p);
   ctx->launches++;
   BEM_CUDA(ctx, cudaGetLastError());
   const size_t smem = (size_t)jc * m.ng * sizeof(double4);

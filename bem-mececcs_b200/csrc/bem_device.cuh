@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "cexp.cuh"
+
 namespace bem {
 
 // Status words in device memory (ctx->d_status[]).
@@ -81,60 +83,68 @@ __device__ __forceinline__ zf crcp(zf z) {
   float s = __frcp_rn(fmaf(z.re, z.re, z.im * z.im));
   return {z.re * s, -z.im * s};
 }
-// exp(z) * scale.
-__device__ __forceinline__ zd cexp_scaled(zd z, double scale) {
-  double s, c;
-  sincos(z.im, &s, &c);
-  double e = exp(z.re) * scale;
-  return {e * c, e * s};
-}
-__device__ __forceinline__ zf cexp_scaled(zf z, float scale) {
-  float s, c;
-  sincosf(z.im, &s, &c);
-  float e = expf(z.re) * scale;
-  return {e * c, e * s};
-}
 __device__ __forceinline__ double cabs1(zd z) { return fabs(z.re) + fabs(z.im); }
 __device__ __forceinline__ float cabs1(zf z) { return fabsf(z.re) + fabsf(z.im); }
 
 // Frequency constants of the Stokes solution, Solfund.for:29-35.
-template <typename R>
 struct StokesConsts {
-  cpx<R> zkp, zks;   // -i w / cp, -i w / cs
-  cpx<R> zc2;        // (cs/cp)^2
-  cpx<R> zc1m2;      // (cp/cs)^2 - 2
-  cpx<R> zc0;        // 1 / (4 pi zge)
-  R inv4pi;
-  cpx<R> izkp, izks; // 1 / zkp, 1 / zks: 1 / (zk r) = (1 / zk) (1 / r), no division per point
+  zd zkp, zks;      // -i w / cp, -i w / cs
+  zd zc2;           // (cs/cp)^2
+  zd zc1m2;         // (cp/cs)^2 - 2
+  zd zc0;           // 1 / (4 pi zge)
+  double inv4pi;
+  zd izkp, izks;    // 1 / zkp, 1 / zks: 1 / (zk r) = (1 / zk) (1 / r), no division per point
+  zd izkp2, izks2;  // their squares
+  int damped;       // the wave numbers have a real part: exp of it is needed
 };
 
 // The radial functions of the Stokes solution at distance r (inverse ir),
-// Solfund.for:36-49: returns FHI, CAPPA, AA, BB, CC.
-template <typename R>
+// Solfund.for:36-49: FHI, CAPPA, AA, BB / 2, CC, and the terms they are built
+// from.  With E = exp(zk r) / r (times zc2 for the P wave),
+//   q = 1/(zk r)^2 - 1/(zk r),  S = Es - Ep,  Q = qs Es - qp Ep,
+//   W = zks Es,  V = zkp Ep
+// the reference's expressions are
+//   FHI = Es + Q            CAPPA = S + 3 Q
+//   AA = W - (2 CAPPA + Es)/r
+//   BB = 2 (V - W + (5 CAPPA + S)/r)
+//   CC = zc1m2 (V - Ep/r) - 2 CAPPA/r
+// (in AA + BB/2 - 3 CAPPA/r the S wave cancels, and V - Ep/r is the
+// derivative of Ep).  56 FP64 operations where term by term they take 125;
+// the FP64 pipe bounds the kernels that evaluate them.
 struct StokesRadial {
-  cpx<R> fhi, cappa, aa, bb, cc;
+  zd fhi, cappa, aa, bbh, cc;
+  zd es, ep, s, w, v, d, cr;  // d = V - Ep/r, cr = CAPPA/r
+  zd q;                       // Q
 };
 
-template <typename R>
-__device__ __forceinline__ StokesRadial<R> stokes_radial(const StokesConsts<R>& k, R r, R ir) {
-  cpx<R> zzs = k.zks * r, zzp = k.zkp * r;
-  cpx<R> es = cexp_scaled(zzs, ir);           // exp(zzs) / r
-  cpx<R> ep = cexp_scaled(zzp, ir) * k.zc2;   // zc2 exp(zzp) / r
-  cpx<R> izs = k.izks * ir, izp = k.izkp * ir;
-  cpx<R> izs2 = izs * izs, izp2 = izp * izp;
-  const R one = R(1), two = R(2), three = R(3), four = R(4), nine = R(9);
-  StokesRadial<R> s;
-  s.fhi = (one + izs2 - izs) * es - (izp2 - izp) * ep;
-  s.cappa = (one + three * izs2 - three * izs) * es - (one + three * izp2 - three * izp) * ep;
-  cpx<R> fhidr = ((-two + zzs + three * izs - three * izs2) * es -
-                  (-one + three * izp - three * izp2) * ep) * ir;
-  cpx<R> cappadr = ((zzs - four + nine * izs - nine * izs2) * es -
-                    (zzp - four + nine * izp - nine * izp2) * ep) * ir;
-  cpx<R> cr = s.cappa * ir;
-  s.aa = fhidr - cr;
-  s.bb = four * cr - two * cappadr;
-  s.cc = k.zc1m2 * (s.aa + R(0.5) * s.bb - three * cr) - two * cr;
-  return s;
+__device__ __forceinline__ StokesRadial stokes_radial(const StokesConsts& k, const CexpTable& tab, double r, double ir) {
+  StokesRadial o;
+  const double2 e0 = cexp_tab(tab, k.zks.re * r, k.zks.im * r, ir, k.damped);
+  const double2 e1 = cexp_tab(tab, k.zkp.re * r, k.zkp.im * r, ir, k.damped);
+  o.es = zd{e0.x, e0.y};
+  o.ep = zd{e1.x, e1.y} * k.zc2;
+  const zd qs{fma(k.izks2.re, ir, -k.izks.re) * ir, fma(k.izks2.im, ir, -k.izks.im) * ir};
+  const zd qp{fma(k.izkp2.re, ir, -k.izkp.re) * ir, fma(k.izkp2.im, ir, -k.izkp.im) * ir};
+  o.q = qs * o.es;
+  cfma(o.q, -qp, o.ep);
+  o.s = o.es - o.ep;
+  o.fhi = o.es + o.q;
+  o.cappa = o.s;
+  cfma(o.cappa, o.q, 3.0);
+  o.w = k.zks * o.es;
+  o.v = k.zkp * o.ep;
+  o.cr = o.cappa * ir;
+  o.d = o.v;
+  cfma(o.d, o.ep, -ir);
+  o.aa = o.w;
+  cfma(o.aa, o.cr, -2.0);
+  cfma(o.aa, o.es, -ir);
+  o.bbh = o.v - o.w;
+  cfma(o.bbh, o.cr, 5.0);
+  cfma(o.bbh, o.s, ir);
+  o.cc = o.cr * -2.0;
+  cfma(o.cc, k.zc1m2, o.d);
+  return o;
 }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {

@@ -272,7 +272,7 @@ int launch_static(bem_ctx* ctx, const double c[4], int compute_gest, double* hes
 int launch_dynamic(bem_ctx* ctx, const double zge[2], const double zcs[2], const double zcp[2],
                    const double c[4], double fr, int flags);
 // Solfund.for:29-35 constants of one frequency (assembly.cu).
-StokesConsts<double> make_consts(const double zge[2], const double zcs[2], const double zcp[2], double fr);
+StokesConsts make_consts(const double zge[2], const double zcs[2], const double zcp[2], double fr);
 // Interior displacements (and stresses when zssol is non-null) on the device (interior.cu).
 int interior_points(bem_ctx* ctx, const double zge[2], const double zcs[2], const double zcp[2], double rho,
                     double fr, int l, const double* cxi, const double* cyi, const double* czi, const double* disp,

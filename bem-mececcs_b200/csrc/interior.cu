@@ -11,12 +11,17 @@
 // tractions after the un-swap.
 //
 // One thread per (interior point, boundary element): the NPG^2 Gauss points
-// of the element (the per-mesh table of k_geometry) are visited once, and at
-// every Gauss point U, T, ZD and ZS are contracted with the element's
-// tractions and displacements straight away (algebraically the reference's
-// sum of element matrices times the boundary vectors; ZD and ZS contract to
-// tensors symmetric in (i, j), so 6 stress components are accumulated).  A
-// CTA reduces its 128 elements in a fixed order and writes one partial per
+// of the element (the per-mesh table of k_geometry) are visited once.  The
+// boundary values t, u and the normal n are constant on the element, so the
+// sums over the Gauss points keep only what varies: the coefficients of t_i,
+// u_i, n_i and rd_i in the displacement (6 complex sums) and of rd_i rd_j,
+// rd_i t_j, rd_i u_j, rd_i n_j, u_i n_j and the identity in the symmetric
+// stress (17); the vectors are multiplied in once per element.  That and the
+// radial functions of bem_device.cuh take about 350 FP64 operations per point
+// where contracting every tensor at every point took some 900; the FP64 pipe
+// bounds the kernel (960 elements x 1000 points, NPG = 4, with stresses:
+// 1078 us before).  A
+// CTA reduces its 64 elements in a fixed order and writes one partial per
 // (point, element chunk); k_interior_reduce sums the chunks in order, so the
 // result does not depend on scheduling.
 #include <cuda_runtime.h>
@@ -31,7 +36,7 @@ namespace bem {
 
 namespace {
 
-constexpr int kIntThreads = 128;  // boundary elements per CTA, one per thread
+constexpr int kIntThreads = 64;   // boundary elements per CTA, one per thread (128 left more of the last CTA idle)
 constexpr int kIntOut = 12;       // 3 displacement + 9 stress components
 constexpr int kIntAcc = 9;        // 3 displacement + 6 symmetric stress components
 
@@ -42,7 +47,7 @@ struct InteriorParams {
   const double4* pts;  // [l] interior points
   const double2* u;    // [3nbe] boundary displacements
   const double2* t;    // [3nbe] boundary tractions
-  StokesConsts<double> kc;
+  StokesConsts kc;
   zd zmu, lm;          // shear modulus ZGE, and lambda / mu
   double2* part;       // [l][chunks][12]
 };
@@ -59,6 +64,9 @@ __host__ __device__ constexpr int sidx(int i, int j) {
 
 __global__ void __launch_bounds__(kIntThreads) k_interior(InteriorParams p) {
   __shared__ zd s_red[kIntThreads / 32][kIntAcc];
+  __shared__ CexpTable tab;
+  cexp_table_fill(tab);
+  __syncthreads();
   const int K = blockIdx.y;
   const int J = blockIdx.x * kIntThreads + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -67,7 +75,7 @@ __global__ void __launch_bounds__(kIntThreads) k_interior(InteriorParams p) {
   for (int i = 0; i < kIntAcc; ++i) acc[i] = zd{0.0, 0.0};
 
   if (J < p.nbe) {
-    const StokesConsts<double>& kc = p.kc;
+    const StokesConsts& kc = p.kc;
     const double4 P = p.pts[K];
     const double4 nv = p.eta[J];
     const double n[3] = {nv.x, nv.y, nv.z};
@@ -81,83 +89,151 @@ __global__ void __launch_bounds__(kIntThreads) k_interior(InteriorParams p) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) cfma(un, u[i], n[i]);
     const double4* q = p.gq + (size_t)J * p.ng;
+    // displacement: sums of FHI, AA dr/dn, AA (rd.u), and the two rd_i
+    // coefficients CAPPA (rd.t) and BB dr/dn (rd.u) + CC (n.u)
+    zd sf{0.0, 0.0}, sa{0.0, 0.0}, sb{0.0, 0.0}, sk[3], sc[3];
+    // stress: c4 (rd.t), c5 dr/dn (rd.u) + c9 (n.u) with rd_i rd_j; c3, c6
+    // dr/dn, c6 (rd.u) with rd_i; c12; the identity's coefficient
+    zd sp[6], s3[3], s6[3], s7[3], s12{0.0, 0.0}, sd{0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) sk[i] = sc[i] = s3[i] = s6[i] = s7[i] = zd{0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) sp[i] = zd{0.0, 0.0};
+    const zd mu4 = p.zmu * kc.inv4pi;
     for (int g = 0; g < p.ng; ++g) {
       const double4 qq = q[g];
       const double r1 = qq.x - P.x, r2 = qq.y - P.y, r3 = qq.z - P.z;
       const double rr = fma(r1, r1, fma(r2, r2, r3 * r3));
-      const double ir = rsqrt(rr);  // r and 1/r from one rsqrt
+      const double ir = rsqrt_fast(rr);  // r and 1/r from one reciprocal square root
       const double r = rr * ir;
       const double rd[3] = {r1 * ir, r2 * ir, r3 * ir};
       const double drn = rd[0] * n[0] + rd[1] * n[1] + rd[2] * n[2];
       const double wt = qq.w;
-      // Radial functions, Solfund.for:36-49 (as stokes_radial) and the
-      // second derivatives of Sigmaec.for, with zzs = -k2 r, zzp = -k1 r.
-      const zd zzs = kc.zks * r, zzp = kc.zkp * r;
-      const zd es = cexp_scaled(zzs, ir);           // exp(zzs) / r
-      const zd ep = cexp_scaled(zzp, ir) * kc.zc2;  // (cs/cp)^2 exp(zzp) / r
-      const zd izs = kc.izks * ir, izp = kc.izkp * ir;
-      const zd izs2 = izs * izs, izp2 = izp * izp;
-      const zd fhi = (1.0 + izs2 - izs) * es - (izp2 - izp) * ep;
-      const zd cappa = (1.0 + 3.0 * izs2 - 3.0 * izs) * es - (1.0 + 3.0 * izp2 - 3.0 * izp) * ep;
-      const zd fhidr = ((-2.0 + zzs + 3.0 * izs - 3.0 * izs2) * es - (-1.0 + 3.0 * izp - 3.0 * izp2) * ep) * ir;
-      const zd cappadr = ((zzs - 4.0 + 9.0 * izs - 9.0 * izs2) * es - (zzp - 4.0 + 9.0 * izp - 9.0 * izp2) * ep) * ir;
-      const zd cr = cappa * ir;
-      const zd aa = fhidr - cr;
-      const zd bb = 4.0 * cr - 2.0 * cappadr;
-      const zd cc = kc.zc1m2 * (aa + 0.5 * bb - 3.0 * cr) - 2.0 * cr;
-      zd rt{0.0, 0.0}, ru{0.0, 0.0};
+      const StokesRadial s = stokes_radial(kc, tab, r, ir);
+      zd rt = t[0] * rd[0], ru = u[0] * rd[0];
+      cfma(rt, t[1], rd[1]);
+      cfma(rt, t[2], rd[2]);
+      cfma(ru, u[1], rd[1]);
+      cfma(ru, u[2], rd[2]);
+      const zd rud = ru * drn;
+      const double w3[3] = {wt * rd[0], wt * rd[1], wt * rd[2]};
+      cfma(sf, s.fhi, wt);
+      cfma(sa, s.aa, wt * drn);
+      cfma(sb, s.aa * ru, wt);
+      const zd kt = s.cappa * rt;
+      zd bc = s.cc * un;
+      cfma(bc, s.bbh * 2.0, rud);
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        cfma(rt, t[i], rd[i]);
-        cfma(ru, u[i], rd[i]);
-      }
-      // Displacements: U(i,:) . t - T(i,:) . u   (Solfund.for:50-60 layouts)
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const zd ug = kc.zc0 * (fhi * t[i] - cappa * (rd[i] * rt));
-        const zd th = kc.inv4pi * (aa * (drn * u[i] + n[i] * ru) + bb * (rd[i] * drn * ru) + cc * (rd[i] * un));
-        cfma(acc[i], ug - th, wt);
+        cfma(sk[i], kt, w3[i]);
+        cfma(sc[i], bc, w3[i]);
       }
       if (p.want_stress) {
+        // SIGMAEC's coefficients (src/Sigmaec.for:96-160).  With D = V - Ep/r
+        // (the derivative of Ep) the second derivatives of the radial
+        // functions enter only through
+        //   FHI'' = zks W - 3 W/r + V/r + (7 Es - 5 Ep + 12 Q)/r^2
+        //   CAPPA'' = zks W - zkp V - 5 (W - V)/r + (17 S + 36 Q)/r^2
+        // and the dilatational terms reduce to lm D and lm zkp V:
+        //   c2 = lm D, c8 = 3 lm D/r - lm zkp V, c10 = 4 CAPPA/r^2 - 4 lm D/r,
+        //   c11 = -lm^2 zkp V.
         const double ir2 = ir * ir;
-        const zd zs2 = zzs * zzs, zp2 = zzp * zzp;
-        const zd fhidrr = ((12.0 * izs2 - 12.0 * izs + 7.0 - 3.0 * zzs + zs2) * es -
-                           (12.0 * izp2 - 12.0 * izp + 5.0 - zzp) * ep) * ir2;
-        const zd cappadrr = ((36.0 * izs2 - 36.0 * izs + 17.0 - 5.0 * zzs + zs2) * es -
-                             (36.0 * izp2 - 36.0 * izp + 17.0 - 5.0 * zzp + zp2) * ep) * ir2;
-        const zd lm = p.lm;
-        const zd cr2 = cappa * ir2, fr1 = fhidr * ir, cr1 = cappadr * ir;
-        const zd c1 = 2.0 * cr;
-        const zd c2 = lm * (fhidr - cappadr - c1);
-        const zd c3 = fhidr - cr;
-        const zd c4 = 2.0 * (cappadr - c1);
-        const zd c5 = 4.0 * (cappadrr - 5.0 * cr1 + 8.0 * cr2);
-        const zd c6 = fhidrr - fr1 - 3.0 * cr1 + 6.0 * cr2;
-        const zd c7 = 2.0 * cr1 - 4.0 * cr2;
-        const zd c8 = lm * (cappadrr + cr1 - 4.0 * cr2 - fhidrr + fr1);
-        const zd c9 = 2.0 * (c7 + c8);
-        const zd c10 = 4.0 * cr2 + 4.0 * lm * (cr1 + 2.0 * cr2 - fr1);
-        const zd c11 = (lm * lm) * (cappadrr + 4.0 * cr1 + 2.0 * cr2 - fhidrr - 2.0 * fr1);
-        const zd c12 = 2.0 * (fr1 - cr2);
-        const zd c12a = c1 - c2, c1011 = c10 + c11;
-        const zd mu4 = p.zmu * kc.inv4pi;
+        const zd cr = s.cr, cr2 = cr * ir;
+        const zd wv = s.w - s.v, ksw = kc.zks * s.w, kpv = kc.zkp * s.v;
+        zd cdr = wv;  // CAPPA' = W - V - (3 CAPPA + S)/r
+        cfma(cdr, cr, -3.0);
+        cfma(cdr, s.s, -ir);
+        zd fdr = s.w;  // FHI' = W - (CAPPA + Es)/r
+        cfma(fdr, cr, -1.0);
+        cfma(fdr, s.es, -ir);
+        const zd fr1 = fdr * ir, cr1 = cdr * ir;
+        zd f2 = ksw;
+        cfma(f2, s.w, -3.0 * ir);
+        cfma(f2, s.v, ir);
+        zd t2 = s.es * 7.0;
+        cfma(t2, s.ep, -5.0);
+        cfma(t2, s.q, 12.0);
+        cfma(f2, t2, ir2);
+        zd k2 = ksw - kpv;
+        cfma(k2, wv, -5.0 * ir);
+        zd t3 = s.s * 17.0;
+        cfma(t3, s.q, 36.0);
+        cfma(k2, t3, ir2);
+        const zd ld = p.lm * s.d, lv = p.lm * kpv;
+        const zd c3 = s.aa;                 // FHI' - CAPPA/r
+        zd c4 = cdr * 2.0;
+        cfma(c4, cr, -4.0);
+        zd c5 = k2 * 4.0;
+        cfma(c5, cr1, -20.0);
+        cfma(c5, cr2, 32.0);
+        zd c6 = f2 - fr1;
+        cfma(c6, cr1, -3.0);
+        cfma(c6, cr2, 6.0);
+        zd c9 = cr1 * 4.0;                  // 2 (c7 + c8), c7 = 2 CAPPA'/r - 4 CAPPA/r^2
+        cfma(c9, cr2, -8.0);
+        cfma(c9, ld, 6.0 * ir);
+        cfma(c9, lv, -2.0);
+        zd c1011 = cr2 * 4.0;
+        cfma(c1011, ld, -4.0 * ir);
+        cfma(c1011, -p.lm, lv);
+        zd c12 = fr1 * 2.0;
+        cfma(c12, cr2, -2.0);
+        zd c12a = cr * 2.0;                 // c1 - c2
+        c12a = c12a - ld;
+        // rd_i rd_j: c4 (rd.t) / 4 pi - mu/(4 pi) (c5 dr/dn (rd.u) + c9 (n.u))
+        zd h = c5 * rud;
+        cfma(h, c9, un);
+        zd pij = (c4 * rt) * kc.inv4pi;
+        cfma(pij, -mu4, h);
+        cfma(sp[0], pij, w3[0] * rd[0]);
+        cfma(sp[1], pij, w3[0] * rd[1]);
+        cfma(sp[2], pij, w3[0] * rd[2]);
+        cfma(sp[3], pij, w3[1] * rd[1]);
+        cfma(sp[4], pij, w3[1] * rd[2]);
+        cfma(sp[5], pij, w3[2] * rd[2]);
+        const zd c6d = c6 * drn, c6u = c6 * ru;
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = i; j < 3; ++j) {
-            const double rij = rd[i] * rd[j];
-            // sum_k t_k ZD(k,i,j)
-            zd d = c4 * (rij * rt) - c3 * (t[j] * rd[i] + t[i] * rd[j]);
-            if (i == j) d = d + c12a * rt;
-            d = kc.inv4pi * d;
-            // sum_k u_k ZS(k,i,j)
-            zd s = drn * (c5 * (rij * ru) - c6 * (u[j] * rd[i] + u[i] * rd[j])) + c9 * (rij * un) -
-                   c6 * ((rd[i] * n[j] + rd[j] * n[i]) * ru) - c12 * (u[i] * n[j] + u[j] * n[i]);
-            if (i == j) s = s + c9 * (drn * ru) + c1011 * un;
-            s = mu4 * s;
-            cfma(acc[3 + sidx(i, j)], d - s, wt);
-          }
+        for (int i = 0; i < 3; ++i) {
+          cfma(s3[i], c3, w3[i]);
+          cfma(s6[i], c6d, w3[i]);
+          cfma(s7[i], c6u, w3[i]);
+        }
+        cfma(s12, c12, wt);
+        zd id = c9 * rud;
+        cfma(id, c1011, un);
+        zd di = (c12a * rt) * kc.inv4pi;
+        cfma(di, -mu4, id);
+        cfma(sd, di, wt);
       }
+    }
+    // Displacements: U(i,:) . t - T(i,:) . u   (Solfund.for:50-60 layouts)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      zd ug = sf * t[i] - sk[i];
+      zd th = sc[i];
+      cfma(th, sa, u[i]);
+      cfma(th, sb, n[i]);
+      acc[i] = kc.zc0 * ug - kc.inv4pi * th;
+    }
+    if (p.want_stress) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = i; j < 3; ++j) {
+          zd d = s3[i] * t[j];  // c3 (t_j rd_i + t_i rd_j)
+          cfma(d, s3[j], t[i]);
+          zd m = s6[i] * u[j];  // c6 dr/dn (u_j rd_i + u_i rd_j) + c6 (rd.u) (rd_i n_j + rd_j n_i)
+          cfma(m, s6[j], u[i]);
+          cfma(m, s7[i], n[j]);
+          cfma(m, s7[j], n[i]);
+          zd un2 = u[i] * n[j];  // c12 (u_i n_j + u_j n_i)
+          cfma(un2, u[j], n[i]);
+          cfma(m, s12, un2);
+          zd a = sp[sidx(i, j)] - kc.inv4pi * d;
+          cfma(a, mu4, m);
+          if (i == j) a = a + sd;
+          acc[3 + sidx(i, j)] = a;
+        }
     }
   }
   // CTA reduction in a fixed order: warp tree, then the 4 warps in order.
