@@ -3336,6 +3336,165 @@ __global__ void __launch_bounds__(256) k_trsv_f32(const __grid_constant__ CUtens
 #include "panel.cuh"
 
 // ---------------------------------------------------------------------------
+// FP64 row interchanges + U12 of one panel on columns [c0, ncols) of problem
+// blockIdx.y, on the DMMA units: tiles of 8 * NQ columns, warp m holding rows
+// 8m..8m+7 of the tile in registers.  The panel rows are gathered by the
+// panel's list and the displaced rows copied; PRE first subtracts the previous
+// panel's deferred product (its L at this panel's rows, its U rows of the
+// tile); then U12 = L11^-1 B block by block: warp b applies the inverse of its
+// 8 x 8 diagonal block (formed once per CTA) and every later warp subtracts
+// L(., b) X_b.
+//
+// Latency bounds it (a few microseconds of flops per launch even at 6480
+// columns), so tiles are narrow: at 8 columns a 720-unknown system's launches
+// spread over as many SMs as it has tiles.  The substitution kernel it
+// replaces (a column per warp, a shuffle chain of 64 to 128 steps) took 31 us
+// with PRE and 15 us without at n = 720, 63 us at n = 6480.
+// ---------------------------------------------------------------------------
+constexpr int kLf64Lp = 66;  // pitch of L by columns: conflict-free A fragments
+constexpr int kLf64Bp = 68;  // pitch of the tiles [column][row]: conflict-free B fragments
+
+template <int NQ>
+constexpr size_t laswp_f64_smem(bool pre) {
+  return ((size_t)(pre ? 2 : 1) * 64 * kLf64Lp + (size_t)(pre ? 2 : 1) * 8 * NQ * kLf64Bp + 8 * 8 * 8) * sizeof(double2);
+}
+
+template <bool PRE, int NQ>
+__global__ void __launch_bounds__(256) k_laswp_f64(double2* Abase, size_t lda, size_t bstride, int k, int w, int c0,
+                                                   int ncols, const int* __restrict__ perm, int perm_stride, int kprev,
+                                                   int wprev) {
+  constexpr int NC = 8 * NQ;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  zd* const s_L = reinterpret_cast<zd*>(smem_raw);              // [64][kLf64Lp] L11 by columns
+  zd* const s_b = s_L + 64 * kLf64Lp;                           // [NC][kLf64Bp] the tile, then X
+  zd* const s_inv = s_b + NC * kLf64Bp;                         // [8][8 columns][8 rows] inverse diagonal blocks
+  zd* const s_Lb = s_inv + 8 * 64;                              // PRE: the previous panel's L at this panel's rows
+  zd* const s_u = s_Lb + 64 * kLf64Lp;                          // PRE: [NC][kLf64Bp] its U rows of the tile
+  __shared__ int s_src[64], s_xd[64], s_xs[64];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  double2* const A = Abase + (size_t)blockIdx.y * bstride;
+  const int* pl = perm + (size_t)blockIdx.y * perm_stride;
+  const int count = pl[0], nx = max(0, count - w);
+  if (tid < 64) {
+    s_src[tid] = tid < w ? pl[2 + 2 * tid] : 0;
+    const int e = w + tid;
+    s_xd[tid] = e < count ? pl[1 + 2 * e] : -1;
+    s_xs[tid] = e < count ? pl[2 + 2 * e] : 0;
+  }
+  __syncthreads();
+  // L11 (strict lower part; the rest and everything past w is zero) and Lb
+  for (int i = tid; i < 64 * 64; i += 256) {
+    const int r = i & 63, c = i >> 6;
+    const bool ok = r < w && c < r;
+    cp_async16(&s_L[c * kLf64Lp + r], ok ? &A[(size_t)(k + c) * lda + k + r] : A, ok);
+    if (PRE) {
+      const bool okb = r < w && c < wprev;
+      cp_async16(&s_Lb[c * kLf64Lp + r], okb ? &A[(size_t)(kprev + c) * lda + s_src[r]] : A, okb);
+    }
+  }
+  cp_async_commit();
+  const int ntiles = (ncols - c0 + NC - 1) / NC;
+  bool first = true;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int cb = c0 + tile * NC, tw = min(NC, ncols - cb);
+    zd xv[2 * NQ];  // displaced rows, loaded before any row is overwritten
+#pragma unroll
+    for (int u = 0; u < 2 * NQ; ++u) {
+      const int i = tid & 63, c = (tid >> 6) + 4 * u;
+      const bool ok = c < tw && i < w;
+      cp_async16(&s_b[c * kLf64Bp + i], ok ? &A[(size_t)(cb + c) * lda + s_src[i]] : A, ok);
+      if (PRE) {
+        const bool oku = c < tw && i < wprev;
+        cp_async16(&s_u[c * kLf64Bp + i], oku ? &A[(size_t)(cb + c) * lda + kprev + i] : A, oku);
+      }
+      xv[u] = i < nx && c < tw ? ldc<double>(&A[(size_t)(cb + c) * lda + s_xs[i]]) : zd{0.0, 0.0};
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    if (first) {  // inverse of diagonal block `warp`, lane = column
+      first = false;
+      if (lane < 8) {
+        zd x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = zd{i == lane ? 1.0 : 0.0, 0.0};
+#pragma unroll
+        for (int t = 0; t < 7; ++t)
+#pragma unroll
+          for (int i = t + 1; i < 8; ++i) cfms(x[i], s_L[(8 * warp + t) * kLf64Lp + 8 * warp + i], x[t]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s_inv[warp * 64 + lane * 8 + i] = x[i];
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int u = 0; u < 2 * NQ; ++u) {
+      const int i = tid & 63, c = (tid >> 6) + 4 * u;
+      if (i < nx && c < tw) stc<double>(&A[(size_t)(cb + c) * lda + s_xd[i]], xv[u]);
+    }
+    const int m0 = 8 * warp;
+    double re[NQ][2], im[NQ][2];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const zd z = s_b[(8 * q + 2 * t4 + e) * kLf64Bp + m0 + g];
+        re[q][e] = z.re;
+        im[q][e] = z.im;
+      }
+    // (re, im) -= M(m0.., k0..k0+3) T(k0..k0+3, .): one K step of the product
+    auto step = [&](zd a, const zd* t) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const zd y = t[(8 * q + g) * kLf64Bp];
+        dmma(re[q][0], re[q][1], -a.re, y.re);
+        dmma(im[q][0], im[q][1], -a.re, y.im);
+        dmma(re[q][0], re[q][1], a.im, y.im);
+        dmma(im[q][0], im[q][1], -a.im, y.re);
+      }
+    };
+    if (PRE)
+#pragma unroll 4
+      for (int kk = 0; kk < wprev; kk += 4) step(s_Lb[(kk + t4) * kLf64Lp + m0 + g], s_u + kk + t4);
+    __syncthreads();  // every warp has its rows of the tile in registers
+    const int nblk = (w + 7) / 8;
+    for (int b = 0; b < nblk; ++b) {
+      if (warp == b) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            s_b[(8 * q + 2 * t4 + e) * kLf64Bp + m0 + g] = zd{re[q][e], im[q][e]};
+            re[q][e] = im[q][e] = 0.0;
+          }
+        __syncwarp();
+#pragma unroll
+        for (int kk = 0; kk < 8; kk += 4) {  // X_b = Inv_b B_b (step subtracts, so -Inv)
+          const zd v = s_inv[b * 64 + (kk + t4) * 8 + g];
+          step(-v, s_b + m0 + kk + t4);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) s_b[(8 * q + 2 * t4 + e) * kLf64Bp + m0 + g] = zd{re[q][e], im[q][e]};
+      }
+      __syncthreads();
+      if (warp > b)
+#pragma unroll
+        for (int kk = 0; kk < 8; kk += 4) step(s_L[(8 * b + kk + t4) * kLf64Lp + m0 + g], s_b + 8 * b + kk + t4);
+    }
+#pragma unroll
+    for (int u = 0; u < 2 * NQ; ++u) {
+      const int i = tid & 63, c = (tid >> 6) + 4 * u;
+      if (c < tw && i < w) stc<double>(&A[(size_t)(cb + c) * lda + k + i], s_b[c * kLf64Bp + i]);
+    }
+    __syncthreads();  // the tile's buffers are refilled
+  }
+  cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
 int lu_ensure_workspace(bem_ctx* ctx, int nn, int batch) {
@@ -3771,29 +3930,43 @@ int f64_update_cublas(bem_ctx* ctx, double2* A, size_t lda, size_t bstride, int 
 // k..k+w1+w2-1): the first panel's columns read through the second panel's
 // gather list (count, then dst/src pairs; row dst of C takes L from row src,
 // as k_gemm_f64 with gperm does), the second panel's as they are.  Out:
-// column-major, ld nn - r0, problem b at out + b * ostride.
+// column-major, ld nn - r0, problem b at out + b * ostride.  kGatherCols
+// columns per CTA, all loads in flight (one CTA per 256 rows, a column at a
+// time, took 31 us whatever the size).
+constexpr int kGatherCols = 8;
 __global__ void __launch_bounds__(256) k_gather_l_pair(const double2* __restrict__ Abase, size_t lda, size_t bstride,
                                                        int nn, int k, int w1, int w2, int r0,
                                                        const int* __restrict__ gperm, int gperm_stride,
                                                        double2* __restrict__ out, size_t ostride) {
   __shared__ int s_map[256];
-  const int b = blockIdx.y, tid = threadIdx.x;
+  const int b = blockIdx.z, tid = threadIdx.x;
   const int row0 = r0 + blockIdx.x * 256, r = row0 + tid;
   const double2* A = Abase + (size_t)b * bstride;
   double2* o = out + (size_t)b * ostride;
   const int m = nn - r0;
   s_map[tid] = r;
   __syncthreads();
-  const int* pl = gperm + (size_t)b * gperm_stride;
-  const int cnt = pl[0];
-  for (int e = tid; e < cnt; e += blockDim.x) {
-    const int dst = pl[1 + 2 * e];
-    if (dst >= row0 && dst < row0 + 256) s_map[dst - row0] = pl[2 + 2 * e];
+  const int cb = blockIdx.y * kGatherCols;
+  if (cb < w1) {
+    const int* pl = gperm + (size_t)b * gperm_stride;
+    const int cnt = pl[0];
+    for (int e = tid; e < cnt; e += blockDim.x) {
+      const int dst = pl[1 + 2 * e];
+      if (dst >= row0 && dst < row0 + 256) s_map[dst - row0] = pl[2 + 2 * e];
+    }
   }
   __syncthreads();
   if (r >= nn) return;
   const int src = s_map[tid];
-  for (int c = 0; c < w1 + w2; ++c) o[(size_t)c * m + (r - r0)] = A[(size_t)(k + c) * lda + (c < w1 ? src : r)];
+  double2 t[kGatherCols];
+#pragma unroll
+  for (int u = 0; u < kGatherCols; ++u) {
+    const int c = cb + u;
+    if (c < w1 + w2) t[u] = A[(size_t)(k + c) * lda + (c < w1 ? src : r)];
+  }
+#pragma unroll
+  for (int u = 0; u < kGatherCols; ++u)
+    if (cb + u < w1 + w2) o[(size_t)(cb + u) * m + (r - r0)] = t[u];
 }
 
 void release_cublas(bem_ctx* ctx) {
@@ -3925,14 +4098,14 @@ static int trsv_f32(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, int
   LuWork& L = ctx->lu;
   done = false;
   const int npan = (int)L.panels.size(), nblk = (nn + kTrsvBlk - 1) / kTrsvBlk;
-  // The largest group (at most 64 CTAs per problem) whose CTAs are all
-  // resident; a share is at most 256 rows (one TMA box), so a large batch of
+  // The largest group (at most a CTA per SM, which a 25920-unknown system needs
+  // for its shares to fit a box) whose CTAs are all resident; a share is at most 256 rows (one TMA box), so a large batch of
   // large systems is solved by several launches of fewer problems.
   int group = 0, ldl = 0, sub = batch;
   size_t smem = 0;
   for (int parts = 1; !group && parts <= batch; ++parts) {
     sub = (batch + parts - 1) / parts;
-    for (int g = std::min(64, std::max(1, nblk)); g >= 1; --g) {
+    for (int g = std::min(std::max(64, ctx->num_sms), std::max(1, nblk)); g >= 1; --g) {
       const int per = (nn + g - 1) / g;
       const int l = (per + 3) & ~1;  // rows of a share rounded out to even ends
       const size_t sm = (size_t)kTrsvBlk * l * sizeof(float2) + (size_t)l * sizeof(int) + 128;
@@ -4063,8 +4236,10 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
   const int cs = cluster_size_for(ctx, nn);
   const size_t lsmem = 64 * 64 * es;
   const size_t bsmem = 64 * 64 * es;
-  BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_trsm<R, false>), lsmem));
-  BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_trsm<R, true>), 2 * lsmem));
+  if constexpr (sizeof(R) == 4) {
+    BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_trsm<R, false>), lsmem));
+    BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_trsm<R, true>), 2 * lsmem));
+  }
   BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_backsub<R>), bsmem));
   BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_gemm_f64), kGemmSmem));
   BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_gemm_tf32), kGemmTf32Smem));
@@ -4241,6 +4416,25 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
       int rc = linv_maps(k, w, perm_p, gi, gsize);
       if (rc) return rc;
     }
+    if constexpr (sizeof(R) == 8) {
+      // tiles of 8 columns while they all run at once, else of 16 on
+      // persistent CTAs (one per SM: shared memory)
+      double2* A2 = static_cast<double2*>(A);
+      const int per = std::max(1, ctx->num_sms / batch), nt8 = (cols + 7) / 8;
+      auto launch = [&](auto kern, size_t sm, int tiles) -> int {
+        BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(kern), sm));
+        kern<<<dim3(std::min(tiles, per), batch), 256, sm, ctx->stream>>>(A2, lda, bstride, k, w, c0, ncols, perm_p,
+                                                                          kPermStride, kfirst, k - kfirst);
+        ctx->launches++;
+        BEM_CUDA(ctx, cudaGetLastError());
+        return BEM_OK;
+      };
+      if (nt8 <= per)
+        return pre ? launch(k_laswp_f64<true, 1>, laswp_f64_smem<1>(true), nt8)
+                   : launch(k_laswp_f64<false, 1>, laswp_f64_smem<1>(false), nt8);
+      return pre ? launch(k_laswp_f64<true, 2>, laswp_f64_smem<2>(true), (cols + 15) / 16)
+                 : launch(k_laswp_f64<false, 2>, laswp_f64_smem<2>(false), (cols + 15) / 16);
+    } else {
     // substitution kernel: at most one earlier panel (pairs), deferred everywhere
     const int blocks = std::max(1, std::min((cols + 31) / 32, (4 * ctx->num_sms + batch - 1) / batch));
     if (pre)
@@ -4252,6 +4446,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     ctx->launches++;
     BEM_CUDA(ctx, cudaGetLastError());
     return BEM_OK;
+    }
   };
   for (int k = 0; k < nn;) {
     const int m = nn - k;
@@ -4361,7 +4556,8 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
             BEM_CUDA(ctx, dev_alloc(ctx, &LW.lg, need * sizeof(double2)));
             LW.lg_cap = need;
           }
-          k_gather_l_pair<<<dim3((nn - kG + 255) / 256, batch), 256, 0, ctx->stream>>>(
+          k_gather_l_pair<<<dim3((nn - kG + 255) / 256, (w1 + w2 + kGatherCols - 1) / kGatherCols, batch), 256, 0,
+                            ctx->stream>>>(
               A2, lda, bstride, nn, k, w1, w2, kG, p2, kPermStride, LW.lg, per);
           ctx->launches++;
           BEM_CUDA(ctx, cudaGetLastError());
