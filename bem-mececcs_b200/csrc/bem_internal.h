@@ -96,7 +96,7 @@ struct LuWork {
   unsigned* trsv_ctr = nullptr;  // [kMaxBatch] group barrier counters
   int* pstart = nullptr;         // first row of each panel of the last factorisation, then nn
                                  // (written by the panel kernels)
-  float2* linv = nullptr;        // [batch][64][64] L11^-1 of the current FP32 panel (k_laswp_tc)
+  float* linv = nullptr;         // [batch] L11^-1 and earlier L of the current FP32 panel as fragments (k_laswp_tc)
   size_t linv_bytes = 0;
   int* gmap = nullptr;           // [batch][kGroupMaps][nn] row maps of a panel group (k_l11_inv)
   size_t gmap_bytes = 0;

@@ -2072,15 +2072,20 @@ __global__ void __launch_bounds__(256) k_laswp_trsm(void* Av, size_t lda, size_t
 }
 
 // ---------------------------------------------------------------------------
-// k_laswp_tc: k_laswp_trsm for the FP32 factors on the tensor cores.  Each
-// CTA first loads L11^-1 (k_l11_inv, once per panel), then loops over
-// 64-column tiles of [c0, ncols): the tile's
-// panel rows are gathered (the panel's interchanges), the displaced rows are
-// copied down, PRE subtracts the previous panel's deferred product Lb Uprev,
-// and U12 = L11^-1 B; both products as TF32 mma.sync (FP32 accumulation,
-// complex as four real products): the deferred product in the accuracy class
-// of the trailing update, U12 with split operands (3 x TF32, about FP32).  U12 goes back to A and, packed and rounded to
-// TF32, to the tensor-core operand rows (ure/uim, when given).
+// k_laswp_tc: k_laswp_trsm for the FP32 factors on the tensor cores, on tiles
+// of 32 columns of [c0, ncols): the tile's panel rows are gathered (the
+// panel's interchanges), the displaced rows copied down, PRE subtracts the
+// group's earlier panels' deferred products Lb_j U_j, and U12 = L11^-1 B, both
+// as TF32 mma.sync products (FP32 accumulation, complex as four real ones):
+// the deferred products in the accuracy class of the trailing update, U12 with
+// split operands (3 x TF32, about FP32).  U12 goes back to A and, packed and
+// rounded to TF32, to the tensor-core operand rows (ure/uim, when given).
+//
+// What bounds it is the latency of a tile's loads, not its flops (2.5 ms of
+// tensor time in a 14-problem sweep of 6480 unknowns that spent 13.6 ms here):
+// the matrices come as ready fragments from L1/L2 (k_l11_inv writes them once
+// per panel), so shared memory holds only the tile and the earlier panels' U
+// rows, two CTAs share an SM, and each issues all loads of a tile at once.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
   const unsigned s = smem_u32(smem);
@@ -2101,25 +2106,69 @@ __device__ __forceinline__ void cp_async_wait() {
 constexpr int kLtLd = 68;  // complex pitch of the 64 x 64 shared tiles (conflict-free fragment loads)
 constexpr size_t kLtTile = (size_t)64 * kLtLd * sizeof(float2);
 
-// L11^-1 of the panel at (k, k) (unit lower, w x w, zero-padded to 64 x 64)
-// for k_laswp_tc, once per panel and problem (one CTA each): by 16 x 16
-// diagonal blocks (a warp each, lane = column), then [[X11, 0], [X21, X22]]
-// with X21 = -X22 L21 X11 at 16 and at 32 (one output per thread of 1024);
-// the zero block above the diagonal (rows 0-31, columns 32-63) holds the
-// intermediate L21 X11.  Row-major [64][64] per problem.
-// In a group of gsize panels (panel gi of it, gi >= 0), it also keeps the
-// group's row maps: map j (of the group's panel j < gsize - 1) gives, for a
+// The matrices a panel's k_laswp_tc multiplies by, as the A fragments of
+// mma.m16n8k8 (TF32): [row tile 4][k step 8][re, im][lane 32] of four floats,
+// kLfragMat floats per 64 x 64 matrix; per problem L11^-1 as a TF32 pair hi +
+// lo, then the earlier panels' L at this panel's rows.
+constexpr int kLfragMat = 64 * 64 * 2, kLfragMats = 2 + kGroupMaps;
+__device__ __forceinline__ int lfrag_index(int i, int t, int part) {
+  return (((((i >> 4) * 8 + (t >> 3)) * 2 + part) * 32 + (i & 7) * 4 + (t & 3)) << 2) + ((i >> 3) & 1) + 2 * ((t >> 2) & 1);
+}
+
+// For the panel at (k, k) of width w, once per panel and problem
+// (blockIdx.y).  blockIdx.x = 0: L11^-1 (unit lower, zero-padded to 64 x 64),
+// by 16 x 16 diagonal blocks (a warp each, lane = column), then [[X11, 0],
+// [X21, X22]] with X21 = -X22 L21 X11 at 16 and at 32 (one output per thread
+// of 1024); the zero block above the diagonal (rows 0-31, columns 32-63)
+// holds the intermediate L21 X11.
+// In a group of gsize panels (panel gi of it, gi >= 0) the group's row maps
+// are kept here too: map j (of the group's panel j < gsize - 1) gives, for a
 // position x now, the position the row held after panel j (where L of panel
-// j stores it). Panel gi replays its interchanges on maps j < gi and starts
-// map gi as the identity below its rows.
+// j stores it).  CTA 0 starts map gi as the identity below its rows, CTA
+// j + 1 replays panel gi's interchanges on map j < gi and packs panel j's L
+// at this panel's rows.
 __global__ void __launch_bounds__(1024) k_l11_inv(const float2* __restrict__ Abase, size_t lda, size_t bstride, int k,
-                                                  int w, float2* out, const int* __restrict__ perm, int perm_stride,
+                                                  int w, float* out, const int* __restrict__ perm, int perm_stride,
                                                   int* gmap, int nn, int gi, int gsize) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* s_inv = reinterpret_cast<float2*>(smem_raw);  // [64][kLtLd]
   float2* s_b = s_inv + 64 * kLtLd;                      // [64][kLtLd] L11
-  const int prob = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int prob = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float2* A = Abase + (size_t)prob * bstride;
+  out += (size_t)prob * kLfragMats * kLfragMat;
+  if (blockIdx.x > 0) {  // map j and panel j's L at this panel's rows
+    __shared__ int s_row[64];
+    const int j = blockIdx.x - 1;
+    int* gm = gmap + ((size_t)prob * kGroupMaps + j) * nn;
+    const int* pl = perm + (size_t)prob * perm_stride;
+    const int count = pl[0];  // at most 128 entries: the panel rows, then the displaced ones
+    int val = 0, dst = -1;
+    if (tid < count) {
+      val = gm[pl[2 + 2 * tid]];
+      dst = pl[1 + 2 * tid];
+    }
+    if (tid < 64) s_row[tid] = tid < w ? val : -1;
+    __syncthreads();  // every read before any write
+    if (dst >= 0) gm[dst] = val;
+    const int kj = k - 64 * (gi - j);  // panel j's first column
+    float* s_f = reinterpret_cast<float*>(smem_raw);
+    float2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int idx = tid + q * 1024, i = idx & 63, t = idx >> 6, r = s_row[i];
+      v[q] = r >= 0 ? A[(size_t)(kj + t) * lda + r] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int idx = tid + q * 1024, i = idx & 63, t = idx >> 6;
+      s_f[lfrag_index(i, t, 0)] = __uint_as_float(to_tf32(v[q].x));
+      s_f[lfrag_index(i, t, 1)] = __uint_as_float(to_tf32(v[q].y));
+    }
+    __syncthreads();
+    float4* o = reinterpret_cast<float4*>(out + (size_t)(2 + j) * kLfragMat);
+    for (int idx = tid; idx < kLfragMat / 4; idx += 1024) o[idx] = reinterpret_cast<const float4*>(s_f)[idx];
+    return;
+  }
   // L11 (unit lower, w x w at (k, k)) into registers first: these loads
   // overlap the row maps' dependent loads below
   float2 lv[4];
@@ -2128,20 +2177,9 @@ __global__ void __launch_bounds__(1024) k_l11_inv(const float2* __restrict__ Aba
     const int idx = tid + q * 1024, i = idx & 63, c = idx >> 6;
     lv[q] = (i < w && c < w) ? A[(size_t)(k + c) * lda + k + i] : make_float2(0.f, 0.f);
   }
-  if (gi >= 0) {
-    int* gm = gmap + (size_t)prob * kGroupMaps * nn;
-    const int* pl = perm + (size_t)prob * perm_stride;
-    const int count = pl[0];
-    const int j = tid >> 7, e = tid & 127;  // map j, entry e (at most 128 entries, 3 maps)
-    int val = 0, dst = -1;
-    if (j < gi && j < kGroupMaps && e < count) {
-      val = gm[(size_t)j * nn + pl[2 + 2 * e]];
-      dst = pl[1 + 2 * e];
-    }
-    __syncthreads();  // every read before any write
-    if (dst >= 0) gm[(size_t)j * nn + dst] = val;
-    if (gi < gsize - 1 && gi < kGroupMaps)
-      for (int x = k + w + tid; x < nn; x += blockDim.x) gm[(size_t)gi * nn + x] = x;
+  if (gi >= 0 && gi < gsize - 1 && gi < kGroupMaps) {
+    int* gm = gmap + ((size_t)prob * kGroupMaps + gi) * nn;
+    for (int x = k + w + tid; x < nn; x += blockDim.x) gm[x] = x;
   }
   // L11 into s_b, row-major; s_inv = I (1024 threads, 4 entries each)
 #pragma unroll
@@ -2205,228 +2243,192 @@ __global__ void __launch_bounds__(1024) k_l11_inv(const float2* __restrict__ Aba
   }
   for (int idx = tid; idx < 32 * 32; idx += blockDim.x) at(s_inv, idx >> 5, 32 + (idx & 31)) = make_float2(0.f, 0.f);
   __syncthreads();
-  float2* o = out + (size_t)prob * 64 * 64;
-  for (int idx = tid; idx < 64 * 64; idx += blockDim.x) o[idx] = s_inv[(idx >> 6) * kLtLd + (idx & 63)];
+  // fragments, through the memory of L11 (hi) and the inverse's own (lo)
+  float* s_hi = reinterpret_cast<float*>(s_b);
+  float2 x[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int idx = tid + q * 1024;
+    x[q] = s_inv[(idx >> 6) * kLtLd + (idx & 63)];
+  }
+  __syncthreads();
+  float* s_lo = reinterpret_cast<float*>(s_inv);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int idx = tid + q * 1024, i = idx >> 6, t = idx & 63;
+    const float re = __uint_as_float(to_tf32(x[q].x)), im = __uint_as_float(to_tf32(x[q].y));
+    s_hi[lfrag_index(i, t, 0)] = re;
+    s_hi[lfrag_index(i, t, 1)] = im;
+    s_lo[lfrag_index(i, t, 0)] = __uint_as_float(to_tf32(x[q].x - re));
+    s_lo[lfrag_index(i, t, 1)] = __uint_as_float(to_tf32(x[q].y - im));
+  }
+  __syncthreads();
+  float4* o = reinterpret_cast<float4*>(out);
+  for (int idx = tid; idx < kLfragMat / 4; idx += 1024) {
+    o[idx] = reinterpret_cast<const float4*>(s_hi)[idx];
+    o[kLfragMat / 4 + idx] = reinterpret_cast<const float4*>(s_lo)[idx];
+  }
 }
 
+constexpr int kLtCols = 32;  // columns of a tile
+constexpr size_t kLtColTile = (size_t)kLtCols * kLtLd * sizeof(float2);
+
 template <bool PRE>
-__global__ void __launch_bounds__(256, 1) k_laswp_tc(float2* Abase, size_t lda, size_t bstride, int k, int w, int c0,
+__global__ void __launch_bounds__(256, 2) k_laswp_tc(float2* Abase, size_t lda, size_t bstride, int k, int w, int c0,
                                                      int ncols, const int* __restrict__ perm, int perm_stride,
                                                      float* ure, float* uim, int urows, int ubase, int koff,
-                                                     int kfirst, int nprev, int cdefer, const int* __restrict__ gmap,
-                                                     int nn, const float2* __restrict__ linv, float* lhat, int lrows,
+                                                     int kfirst, int nprev, int cdefer,
+                                                     int nn, const float* __restrict__ lfrag, float* lhat, int lrows,
                                                      int pk_r0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* s_inv = reinterpret_cast<float2*>(smem_raw);  // [64][kLtLd] L11^-1, row-major
-  float2* s_bb = s_inv + 64 * kLtLd;                     // [2][64][kLtLd] tiles (panel rows x columns), two stages
-  float2* s_lb = s_bb + 2 * 64 * kLtLd;                  // PRE: an earlier panel's L at this panel's rows
-  float2* s_upb = s_lb + 64 * kLtLd;                     // PRE: [2][64][kLtLd] that panel's U rows of the tile
-  __shared__ int s_src[64];                              // source row of panel row i
-  __shared__ int s_xd[64], s_xs[64];                     // displaced rows: dst <- src
-  __shared__ int s_nx;
+  float2* const s_b = reinterpret_cast<float2*>(smem_raw);  // [kLtCols][kLtLd] the tile by columns
+  float2* const s_u = s_b + kLtCols * kLtLd;                // PRE: [nprev][kLtCols][kLtLd] the earlier panels' U rows
+  __shared__ int s_src[64];                                 // source row of panel row i
+  __shared__ int s_xd[64], s_xs[64];                        // displaced rows: dst <- src
   const int prob = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float2* A = Abase + (size_t)prob * bstride;
   const int* pl = perm + (size_t)prob * perm_stride;
-  const int count = pl[0];
-  if (tid < 64) s_src[tid] = tid < w ? pl[2 + 2 * tid] : 0;
+  const int count = pl[0], nx = max(0, count - w);
   if (tid < 64) {
+    s_src[tid] = tid < w ? pl[2 + 2 * tid] : 0;
     const int e = w + tid;
     s_xd[tid] = e < count ? pl[1 + 2 * e] : -1;
     s_xs[tid] = e < count ? pl[2 + 2 * e] : 0;
   }
-  if (tid == 0) s_nx = max(0, count - w);
-  // L11^-1 (k_l11_inv) into s_inv by cp.async
-  {
-    const float2* li = linv + (size_t)prob * 64 * 64;
-    for (int idx = tid; idx < 64 * 64; idx += blockDim.x)
-      cp_async8(&s_inv[(idx >> 6) * kLtLd + (idx & 63)], &li[idx], true);
-    cp_async_commit();
-  }
-  __syncthreads();  // s_src
-  // Lb_j(i, t) = L(map_j(k + i), kfirst + 64 j + t): earlier panel j's L at this panel's rows
-  const int* gm = gmap + (size_t)prob * kGroupMaps * nn;
-  auto load_lb_to = [&](float2* dst, int j) {
-    for (int idx = tid; idx < 64 * 64; idx += blockDim.x) {
-      const int i = idx & 63, t = idx >> 6;
-      const bool ok = i < w;
-      cp_async8(&dst[i * kLtLd + t], ok ? &A[(size_t)(kfirst + 64 * j + t) * lda + gm[(size_t)j * nn + k + i]] : A,
-                ok);
-    }
+  __syncthreads();
+  // warp tile: rows [16 * (warp & 3), +16) x columns [16 * (warp >> 2), +16)
+  const int g = lane >> 2, t4 = lane & 3, mrow = 16 * (warp & 3), ncol = 16 * (warp >> 2);
+  // this warp's fragments of matrix m: (m * 4 + row tile) * 8 k steps x 2 parts x 32 lanes
+  const float4* const fr = reinterpret_cast<const float4*>(lfrag + (size_t)prob * kLfragMats * kLfragMat) +
+                           (size_t)(warp & 3) * 8 * 2 * 32 + lane;
+  auto frag = [&](int m, int ks, int part, unsigned (&a)[4]) {
+    const float4 f = __ldg(fr + ((size_t)m * 4 * 8 + ks) * 64 + part * 32);
+    a[0] = __float_as_uint(f.x);
+    a[1] = __float_as_uint(f.y);
+    a[2] = __float_as_uint(f.z);
+    a[3] = __float_as_uint(f.w);
   };
-  auto load_lb = [&](int j) { load_lb_to(s_lb, j); };
-  // earlier panel j's U rows of the tile at cbase (tw columns)
-  auto load_up_to = [&](float2* dst, int j, int cbase, int tw) {
-    const int i = tid & 63, cg = tid >> 6;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int c = cg + 4 * u;
-      cp_async8(&dst[i * kLtLd + c], c < tw ? &A[(size_t)(cbase + c) * lda + kfirst + 64 * j + i] : A, c < tw);
-    }
-  };
-  if (PRE) load_lb(0);
-  cp_async_commit();
-
-  // warp tile: rows [16 * (warp & 3), +16) x columns [32 * (warp >> 2), +32)
-  const int g = lane >> 2, t4 = lane & 3, mrow = 16 * (warp & 3), ncol = 32 * (warp >> 2);
-  // acc += M B for this warp's tile, M (64 x 64) and B (64 x 64) complex in
-  // shared memory; split: each operand as a TF32 pair hi + lo and three
-  // products per real product (hi hi + hi lo + lo hi), about FP32 accuracy.
-  auto zero_acc = [&](float (&pr)[4][4], float (&pi)[4][4]) {
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) pr[nt][e] = pi[nt][e] = 0.f;
-  };
-  auto cproduct = [&](const float2* M, const float2* Bm, float (&pr)[4][4], float (&pi)[4][4], bool split) {
+  // acc += M T for this warp's tile; T by columns in shared memory.  split:
+  // M and T as TF32 pairs hi + lo, three products per real product (hi hi +
+  // hi lo + lo hi), about FP32 accuracy.
+  auto cproduct = [&](int m, const float2* T, float (&pr)[2][4], float (&pi)[2][4], auto split) {
+    constexpr bool kSplit = decltype(split)::value;
 #pragma unroll 2
     for (int ks = 0; ks < 8; ++ks) {
-      const int kc = ks * 8 + t4;
-      const float2 x0 = M[(mrow + g) * kLtLd + kc], x1 = M[(mrow + g + 8) * kLtLd + kc];
-      const float2 x2 = M[(mrow + g) * kLtLd + kc + 4], x3 = M[(mrow + g + 8) * kLtLd + kc + 4];
-      const unsigned ar[4] = {to_tf32(x0.x), to_tf32(x1.x), to_tf32(x2.x), to_tf32(x3.x)};
-      const unsigned ai[4] = {to_tf32(x0.y), to_tf32(x1.y), to_tf32(x2.y), to_tf32(x3.y)};
-      const unsigned an[4] = {ai[0] ^ 0x80000000u, ai[1] ^ 0x80000000u, ai[2] ^ 0x80000000u, ai[3] ^ 0x80000000u};
-      unsigned arl[4], ail[4], anl[4];  // low parts (split)
-      if (split) {
-        const float xr[4] = {x0.x, x1.x, x2.x, x3.x}, xi[4] = {x0.y, x1.y, x2.y, x3.y};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          arl[e] = to_tf32(xr[e] - __uint_as_float(ar[e]));
-          ail[e] = to_tf32(xi[e] - __uint_as_float(ai[e]));
-          anl[e] = ail[e] ^ 0x80000000u;
-        }
+      unsigned ar[4], ai[4], an[4], arl[4], ail[4], anl[4];
+      frag(m, ks, 0, ar);
+      frag(m, ks, 1, ai);
+      if constexpr (kSplit) {
+        frag(m + 1, ks, 0, arl);
+        frag(m + 1, ks, 1, ail);
       }
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const int cb = ncol + nt * 8 + g;
-        const float2 y0 = Bm[kc * kLtLd + cb], y1 = Bm[(kc + 4) * kLtLd + cb];
+      for (int e = 0; e < 4; ++e) {
+        an[e] = ai[e] ^ 0x80000000u;
+        if constexpr (kSplit) anl[e] = ail[e] ^ 0x80000000u;
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const float2* tc = T + (ncol + nt * 8 + g) * kLtLd + ks * 8 + t4;
+        const float2 y0 = tc[0], y1 = tc[4];
         const unsigned br[2] = {to_tf32(y0.x), to_tf32(y1.x)}, bi[2] = {to_tf32(y0.y), to_tf32(y1.y)};
         mma_tf32(pr[nt], ar, br);
-        mma_tf32(pr[nt], an, bi);
         mma_tf32(pi[nt], ar, bi);
+        mma_tf32(pr[nt], an, bi);
         mma_tf32(pi[nt], ai, br);
-        if (split) {
+        if constexpr (kSplit) {
           const unsigned brl[2] = {to_tf32(y0.x - __uint_as_float(br[0])), to_tf32(y1.x - __uint_as_float(br[1]))};
           const unsigned bil[2] = {to_tf32(y0.y - __uint_as_float(bi[0])), to_tf32(y1.y - __uint_as_float(bi[1]))};
           mma_tf32(pr[nt], ar, brl);
-          mma_tf32(pr[nt], an, bil);
           mma_tf32(pi[nt], ar, bil);
+          mma_tf32(pr[nt], an, bil);
           mma_tf32(pi[nt], ai, brl);
           mma_tf32(pr[nt], arl, br);
-          mma_tf32(pr[nt], anl, bi);
           mma_tf32(pi[nt], arl, bi);
+          mma_tf32(pr[nt], anl, bi);
           mma_tf32(pi[nt], ail, br);
         }
       }
     }
   };
-
-  const int ntiles = (ncols - c0 + 63) / 64;
-  // A tile's gathered panel rows into stage st by cp.async (8-byte elements,
-  // zero-filled outside the panel rows and past the last column).
-  // With it, for a deferred tile, the first earlier panel's U rows (and its
-  // Lb again when the tile before used s_lb for a third panel).
-  auto issue = [&](int tile, int st, bool lb0) {
-    if (tile < ntiles) {
-      const int cbase = c0 + tile * 64, tw = min(64, ncols - cbase);
-      float2* b = s_bb + (size_t)st * 64 * kLtLd;
-      const int i = tid & 63, cg = tid >> 6;
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int c = cg + 4 * u;
-        const bool ok = c < tw && i < w;
-        cp_async8(&b[i * kLtLd + c], ok ? &A[(size_t)(cbase + c) * lda + s_src[i]] : A, ok);
-      }
-      if (PRE && cbase >= cdefer) {
-        load_up_to(s_upb + (size_t)st * 64 * kLtLd, 0, cbase, tw);
-        if (lb0) load_lb(0);
-      }
-    }
-    cp_async_commit();
-  };
-  issue(blockIdx.x, 0, false);
-  for (int it = 0;; ++it) {
-    const int tile = blockIdx.x + it * gridDim.x;
-    if (tile >= ntiles) break;
-    const int st = it & 1;
-    const int cbase = c0 + tile * 64, tw = min(64, ncols - cbase);
-    float2* sb = s_bb + (size_t)st * 64 * kLtLd;
-    cp_async_wait<0>();
-    __syncthreads();
-    // displaced rows: their sources, loaded now and stored after the products
-    float2 xv[16];
-    const int nx = s_nx;
+  const int ntiles = (ncols - c0 + kLtCols - 1) / kLtCols;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int cbase = c0 + tile * kLtCols, tw = min(kLtCols, ncols - cbase);
+    const bool defer = PRE && cbase >= cdefer;
+    // every load of the tile in flight at once; the SM's other CTA covers it
     {
       const int i = tid & 63, cg = tid >> 6;
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
+      for (int u = 0; u < kLtCols / 4; ++u) {
         const int c = cg + 4 * u;
-        xv[u] = (i < nx && c < tw) ? A[(size_t)(cbase + c) * lda + s_xs[i]] : make_float2(0.f, 0.f);
+        const bool ok = c < tw && i < w;
+        cp_async8(&s_b[c * kLtLd + i], ok ? &A[(size_t)(cbase + c) * lda + s_src[i]] : A, ok);
       }
     }
-    float pr[4][4], pi[4][4];
-    if (PRE && cbase >= cdefer) {  // B -= sum_j Lb_j Uprev_j: the group's deferred update of these rows
-      // Two operand slots: slot 0 = (s_lb, this stage's U buffer), which the
-      // tile's own loads filled with panel 0's; slot 1 = the other stage's
-      // tile and U buffers, idle until the next tile is issued.  Panel j + 1's
-      // operands load into the other slot while panel j's product runs.
-      float2* const lb0 = s_lb;
-      float2* const lb1 = s_bb + (size_t)(st ^ 1) * 64 * kLtLd;
-      float2* const up0 = s_upb + (size_t)st * 64 * kLtLd;
-      float2* const up1 = s_upb + (size_t)(st ^ 1) * 64 * kLtLd;
-      zero_acc(pr, pi);
-      for (int j = 0; j < nprev; ++j) {
-        const bool odd = j & 1;
-        if (j + 1 < nprev) {
-          load_lb_to(odd ? lb0 : lb1, j + 1);
-          load_up_to(odd ? up0 : up1, j + 1, cbase, tw);
-          cp_async_commit();
-          cp_async_wait<1>();
-        } else {
-          cp_async_wait<0>();
-        }
-        __syncthreads();
-        cproduct(odd ? lb1 : lb0, odd ? up1 : up0, pr, pi, false);
-        __syncthreads();  // slot sl is refilled two panels on
-      }
+    if (defer) {
+      const int i = 2 * lane, cg = warp;
+      for (int j = 0; j < nprev; ++j)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+        for (int u = 0; u < kLtCols / 8; ++u) {
+          const int c = cg + 8 * u;
+          cp_async16(&s_u[(j * kLtCols + c) * kLtLd + i],
+                     c < tw ? &A[(size_t)(cbase + c) * lda + kfirst + 64 * j + i] : A, c < tw);
+        }
+    }
+    cp_async_commit();
+    float2 xv[kLtCols / 4];  // displaced rows: their sources, before any row is overwritten
+    const int xi = tid & 63, xc = tid >> 6;
+#pragma unroll
+    for (int u = 0; u < kLtCols / 4; ++u) {
+      const int c = xc + 4 * u;
+      xv[u] = (xi < nx && c < tw) ? A[(size_t)(cbase + c) * lda + s_xs[xi]] : make_float2(0.f, 0.f);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kLtCols / 4; ++u) {
+      const int c = xc + 4 * u;
+      if (xi < nx && c < tw) A[(size_t)(cbase + c) * lda + s_xd[xi]] = xv[u];
+    }
+    float pr[2][4], pi[2][4];
+    auto zero_acc = [&]() {
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) pr[nt][e] = pi[nt][e] = 0.f;
+    };
+    // element e of n tile nt: row and column in the tile
+    auto at = [&](int nt, int e) -> float2& {
+      return s_b[(ncol + nt * 8 + 2 * t4 + (e & 1)) * kLtLd + mrow + g + ((e >> 1) << 3)];
+    };
+    if (defer) {  // B -= sum_j Lb_j U_j: the group's deferred update of these rows
+      zero_acc();
+      for (int j = 0; j < nprev; ++j) cproduct(2 + j, s_u + (size_t)j * kLtCols * kLtLd, pr, pi, std::false_type{});
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int r = mrow + g + ((e >> 1) << 3), c = ncol + nt * 8 + 2 * t4 + (e & 1);
-          float2& z = sb[r * kLtLd + c];
+          float2& z = at(nt, e);
           z.x -= pr[nt][e];
           z.y -= pi[nt][e];
         }
       __syncthreads();
     }
-    issue(tile + gridDim.x, st ^ 1, nprev >= 3);  // the next tile streams in meanwhile
-    zero_acc(pr, pi);
-    cproduct(s_inv, sb, pr, pi, true);  // U12 = L11^-1 B
-    __syncthreads();                     // every warp has read the tile
+    zero_acc();
+    cproduct(0, s_b, pr, pi, std::true_type{});  // U12 = L11^-1 B
+    __syncthreads();                              // every warp has read the tile
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = mrow + g + ((e >> 1) << 3), c = ncol + nt * 8 + 2 * t4 + (e & 1);
-        sb[r * kLtLd + c] = make_float2(pr[nt][e], pi[nt][e]);
-      }
-    {  // displaced rows get the rows they replaced (all reads of them came first)
-      const int i = tid & 63, cg = tid >> 6;
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int c = cg + 4 * u;
-        if (i < nx && c < tw) A[(size_t)(cbase + c) * lda + s_xd[i]] = xv[u];
-      }
-    }
+      for (int e = 0; e < 4; ++e) at(nt, e) = make_float2(pr[nt][e], pi[nt][e]);
     __syncthreads();
     {  // U12 to A (rows k..k+w-1) and packed K-major TF32 rows
       const int i = tid & 63, cg = tid >> 6;
-#pragma unroll 4
-      for (int u = 0; u < 16; ++u) {
+#pragma unroll
+      for (int u = 0; u < kLtCols / 4; ++u) {
         const int c = cg + 4 * u;
         if (c >= tw) continue;
-        const float2 z = sb[i * kLtLd + c];
+        const float2 z = s_b[c * kLtLd + i];
         if (i < w) A[(size_t)(cbase + c) * lda + k + i] = z;
         if (ure) {
           const size_t row = ((size_t)prob * urows + (cbase + c - ubase)) * kTcKPitch + koff;
@@ -2435,15 +2437,14 @@ __global__ void __launch_bounds__(256, 1) k_laswp_tc(float2* Abase, size_t lda, 
         }
       }
     }
-    __syncthreads();  // this stage is refilled two tiles on
+    __syncthreads();  // the buffers are refilled by the next tile
   }
-  cp_async_wait<0>();
   if (pk_r0 >= 0 && pk_r0 < nn) {
     // this panel's L21 (rows pk_r0..nn-1) packed for the update that follows,
     // at its K slot, 32-row blocks dealt to the CTAs (the tiles' shared memory)
     __shared__ int s_psrc[32];
     __syncthreads();
-    auto tile = reinterpret_cast<float2(*)[33]>(s_bb);
+    auto tile = reinterpret_cast<float2(*)[33]>(s_b);
     float* out = lhat + (size_t)prob * lrows * kTcKPitch;
     const int nblk = (nn - pk_r0 + 31) / 32;
     for (int bi = blockIdx.x; bi < nblk; bi += gridDim.x) {
@@ -4344,7 +4345,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
   // of gsize, the group's row maps (k_l11_inv).
   auto linv_maps = [&](int k, int w, const int* perm_p, int gi, int gsize) -> int {
     LuWork& LW = ctx->lu;
-    const size_t lbytes = (size_t)batch * 64 * 64 * sizeof(float2);
+    const size_t lbytes = (size_t)batch * kLfragMats * kLfragMat * sizeof(float);
     if (LW.linv_bytes < lbytes) {
       dev_free(ctx, LW.linv);
       LW.linv = nullptr;
@@ -4361,8 +4362,8 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
       LW.gmap_bytes = mbytes;
     }
     BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_l11_inv), (2 * kLtTile)));
-    k_l11_inv<<<batch, 1024, 2 * kLtTile, ctx->stream>>>(static_cast<const float2*>(A), lda, bstride, k, w, LW.linv,
-                                                         perm_p, kPermStride, LW.gmap, nn, gi, gsize);
+    k_l11_inv<<<dim3(1 + std::min(std::max(gi, 0), kGroupMaps), batch), 1024, 2 * kLtTile, ctx->stream>>>(
+        static_cast<const float2*>(A), lda, bstride, k, w, LW.linv, perm_p, kPermStride, LW.gmap, nn, gi, gsize);
     ctx->launches++;
     BEM_CUDA(ctx, cudaGetLastError());
     return BEM_OK;
@@ -4387,11 +4388,11 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     if (sizeof(R) == 4 && ctx->laswp_tc) {
       int rc = linv_maps(k, w, perm_p, gi, gsize);
       if (rc) return rc;
-      // one CTA per SM (registers; shared memory for three or six 64 x 64 tiles)
-      const int ntiles = (cols + 63) / 64;
-      const int per = std::max(1, ctx->num_sms / batch);
+      // two CTAs per SM
+      const int ntiles = (cols + kLtCols - 1) / kLtCols;
+      const int per = std::max(1, 2 * ctx->num_sms / batch);
       const int tb = std::min(ntiles, per);
-      const size_t sm = (pre ? 6 : 3) * kLtTile;
+      const size_t sm = (1 + nprev) * kLtColTile;
       float2* A2 = static_cast<float2*>(A);
       LuWork& LW = ctx->lu;
       const int pk = (ure && pack_r0 >= 0) ? pack_r0 : -1;
@@ -4400,12 +4401,12 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
         BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_tc<true>), sm));
         k_laswp_tc<true><<<dim3(tb, batch), 256, sm, ctx->stream>>>(
             A2, lda, bstride, k, w, c0, ncols, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, nprev,
-            cdefer, LW.gmap, nn, LW.linv, lhat, 2 * nn, pk);
+            cdefer, nn, LW.linv, lhat, 2 * nn, pk);
       } else {
         BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_tc<false>), sm));
         k_laswp_tc<false><<<dim3(tb, batch), 256, sm, ctx->stream>>>(
-            A2, lda, bstride, k, w, c0, ncols, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, 0, ncols,
-            LW.gmap, nn, LW.linv, lhat, 2 * nn, pk);
+            A2, lda, bstride, k, w, c0, ncols, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, 0, ncols, nn,
+            LW.linv, lhat, 2 * nn, pk);
       }
       ctx->launches++;
       BEM_CUDA(ctx, cudaGetLastError());
