@@ -113,6 +113,10 @@ struct LuWork {
   float2* tinv = nullptr;        // FP32 solves: inverted diagonal blocks of the last factors
   size_t tinv_bytes = 0;
   bool tinv_valid = false;
+  bool uinv_valid = false;       // k_trsv_cl: tinv holds the U blocks' inverses by columns
+  bool lperm_valid = false;      // ... and the L blocks', and L is in its final row order
+  int* rmap = nullptr;           // [batch][panel + 1][nn] row maps (k_row_maps), then [batch][panel] moved flags
+  size_t rmap_bytes = 0;
   double2* lg = nullptr;         // FP64 panel pairs on cuBLAS: both panels' L, the first gathered
   size_t lg_cap = 0;             // elements
 };

@@ -215,6 +215,7 @@ int bem_ctx_destroy(bem_ctx* ctx) {
   dev_free(ctx, L.barrier);
   dev_free(ctx, L.trsv_w);
   dev_free(ctx, L.tinv);
+  dev_free(ctx, L.rmap);
   dev_free(ctx, L.linv);
   dev_free(ctx, L.gmap);
   dev_free(ctx, L.trsv_ctr);

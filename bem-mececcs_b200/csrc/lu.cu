@@ -3335,6 +3335,7 @@ __global__ void __launch_bounds__(256) k_trsv_f32(const __grid_constant__ CUtens
 }
 
 #include "panel.cuh"
+#include "trsv.cuh"
 
 // ---------------------------------------------------------------------------
 // FP64 row interchanges + U12 of one panel on columns [c0, ncols) of problem
@@ -4094,6 +4095,109 @@ bool make_rows_map(CUtensorMap* m, const void* base, int nn, size_t lda, size_t 
 // memory would not fit, and k_trsv runs instead.
 constexpr size_t kTrsvF32SmemMax = 200 * 1024;
 
+// The cluster form (k_trsv_cl): done = false when the factorisation's panels
+// are not 64 wide, or a CTA's rows, the permutation's tables or a ring of two
+// stages do not fit shared memory, and for systems so tall that a cluster's
+// few SMs read the factors more slowly (57 GB/s each) than the cooperative
+// kernel's steps take (about 6 us): more than 20 blocks a CTA, n > 20500 alone
+// (25920 unknowns: 5.9 ms a solve here, 4 ms there).  The cooperative kernels
+// run instead.  Once L has been put into its final row order only this form
+// may use it.
+static int trsv_cl(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int batch, void* v, size_t vstride,
+                   bool forward, bool& done) {
+  LuWork& L = ctx->lu;
+  done = false;
+  const int npan = (int)L.panels.size(), nb = (nn + 63) / 64;
+  if (npan != nb) return BEM_OK;
+  for (int p = 0; p < npan; ++p)
+    if (L.panels[p].first != 64 * p) return BEM_OK;
+  constexpr size_t kSmem = (size_t)226 * 1024 - 12 * 1024;  // less the kernel's static shared memory
+  if ((size_t)2 * nn * sizeof(int) > kSmem) return BEM_OK;
+  // CTAs per problem: as many as leave every problem's cluster its own SMs
+  int G = std::min(16, cluster_size(ctx));
+  while (G > 1 && (G > nb || G * batch > ctx->num_sms)) G /= 2;
+  const int own = (nb + G - 1) / G;
+  if (own > 20) return BEM_OK;
+  const size_t fixed = (size_t)own * 64 * 5 * sizeof(float2) + 128, stage = (size_t)kTclStage * sizeof(float2);
+  if (fixed + 2 * stage > kSmem) return BEM_OK;
+  const int stages = (int)std::min<size_t>(6, (kSmem - fixed) / stage);
+  CUtensorMap tm;
+  if (!make_rows_map(&tm, A, nn, lda, bstride, batch, 64)) return BEM_OK;
+  auto need = [&](auto*& p, size_t& cap, size_t bytes) -> int {
+    if (cap >= bytes) return BEM_OK;
+    dev_free(ctx, p);
+    p = nullptr;
+    cap = 0;
+    BEM_CUDA(ctx, dev_alloc(ctx, &p, bytes));
+    cap = bytes;
+    return BEM_OK;
+  };
+  int rc = need(L.tinv, L.tinv_bytes, (size_t)batch * (npan + nb) * stage);
+  if (rc) return rc;
+  float2* A2 = static_cast<float2*>(A);
+  constexpr size_t kInvSmem = 2 * kLtTile;
+  BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_tri_inv_cl), kInvSmem));
+  auto invert = [&](int b0, int count) -> int {
+    k_tri_inv_cl<<<dim3(count, batch), 256, kInvSmem, ctx->stream>>>(A2, lda, bstride, nn, npan, b0, npan + nb, L.tinv);
+    ctx->launches++;
+    BEM_CUDA(ctx, cudaGetLastError());
+    return BEM_OK;
+  };
+  if (!L.uinv_valid) {
+    rc = invert(npan, nb);
+    if (rc) return rc;
+    L.uinv_valid = true;
+    L.tinv_valid = false;
+  }
+  if (forward && !L.lperm_valid) {
+    rc = need(L.rmap, L.rmap_bytes, ((size_t)(npan + 1) * nn + npan) * batch * sizeof(int));
+    if (rc) return rc;
+    int* moved = L.rmap + (size_t)(npan + 1) * nn * batch;
+    const size_t msm = (size_t)2 * nn * sizeof(int), psm = (size_t)nn * sizeof(float2);
+    BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_row_maps), msm));
+    BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_lperm), psm));
+    rc = invert(0, npan);
+    if (rc) return rc;
+    k_row_maps<<<batch, 1024, msm, ctx->stream>>>(nn, npan, batch, L.perm, L.rmap, moved);
+    if (npan > 1)
+      k_lperm<<<dim3(npan - 1, 16, batch), 256, psm, ctx->stream>>>(A2, lda, bstride, nn, npan, L.rmap, moved);
+    ctx->launches += 2;
+    BEM_CUDA(ctx, cudaGetLastError());
+    L.lperm_valid = true;
+  }
+  TrsvClArgs t{};
+  t.v = static_cast<float2*>(v);
+  t.vstride = vstride;
+  t.nn = nn;
+  t.nb = nb;
+  t.npan = npan;
+  t.forward = forward ? 1 : 0;
+  t.stages = stages;
+  t.own = own;
+  t.tinv = L.tinv;
+  t.rows = forward ? L.rmap : nullptr;
+  t.status = ctx->d_status;
+  const size_t smem = fixed + (size_t)stages * stage;
+  BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_trsv_cl), smem));
+  BEM_CUDA(ctx, cudaFuncSetAttribute(k_trsv_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(G, batch, 1);
+  cfg.blockDim = dim3(kTclThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = G;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  BEM_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_trsv_cl, tm, t));
+  ctx->launches++;
+  done = true;
+  return BEM_OK;
+}
+
 static int trsv_f32(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, int nn, int batch, void* v,
                     size_t vstride, bool forward, bool& done) {
   LuWork& L = ctx->lu;
@@ -4143,6 +4247,7 @@ static int trsv_f32(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, int
     ctx->launches++;
     BEM_CUDA(ctx, cudaGetLastError());
     L.tinv_valid = true;
+    L.uinv_valid = false;
   }
   TrsvArgs t{};
   t.A = A;
@@ -4190,8 +4295,13 @@ static int trsv_coop(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, in
   if (!L.trsv_ctr) BEM_CUDA(ctx, dev_alloc(ctx, &L.trsv_ctr, kMaxBatch * sizeof(unsigned)));
   if (batch < 1 || batch > kMaxBatch) return fail(ctx, BEM_ERR_ARG, "batch size out of range");
   if constexpr (sizeof(R) == 4) {
-    if (ctx->trsv_inv) {
+    if (ctx->trsv_inv || L.lperm_valid) {
       bool done = false;
+      if (ctx->trsv_ctas == 0 || L.lperm_valid) {
+        const int rc = trsv_cl(ctx, const_cast<void*>(A), lda, bstride, nn, batch, v, vstride, forward, done);
+        if (rc || done) return rc;
+        if (L.lperm_valid) return fail(ctx, BEM_ERR_STATE, "solve with permuted factors does not fit");
+      }
       const int rc = trsv_f32(ctx, A, lda, bstride, nn, batch, v, vstride, forward, done);
       if (rc || done) return rc;
     }
@@ -4249,7 +4359,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     if (rc) return rc;
   }
   L.panels.clear();
-  L.tinv_valid = false;  // the solves' block inverses belong to the previous factors
+  L.tinv_valid = L.uinv_valid = L.lperm_valid = false;  // the solves' data belongs to the previous factors
   const bool tc = sizeof(R) == 4 && ctx->use_tcgen05;
   // Panel width for m remaining rows: the widest of 64/32/16 whose rows fit
   // one cluster, at most 512 rows per CTA (one row per thread); 0 when the
@@ -4698,7 +4808,7 @@ static int lu_solve_vec_t(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int
   BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_fwd_panel<R>), lsmem));
   BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_backsub<R>), lsmem));
   ProfScope ps(ctx, 4, 8.0 * (double)nn * nn * batch, (double)nn * nn * sizeof(cpx<R>) * batch);
-  if (ctx->use_trsv_coop) return trsv_coop<R>(ctx, A, lda, bstride, nn, batch, v, vstride, true);
+  if (ctx->use_trsv_coop || L.lperm_valid) return trsv_coop<R>(ctx, A, lda, bstride, nn, batch, v, vstride, true);
   for (size_t p = 0; p < L.panels.size(); ++p) {
     const int k = L.panels[p].first, w = L.panels[p].second;
     const int* perm_p = L.perm + p * (size_t)batch * kPermStride;

@@ -57,3 +57,25 @@ def test_fp32_panel(nx, ny):
             xm, _ = sol.sweep(freqs, form="mixed", batch=batch, refine=4)
             for i in range(len(freqs)):
                 assert rel(xm[i], xp[i]) < 1e-10, (batch, freqs[i])
+
+
+# 1 to 17 row blocks on clusters of 1 to 16 CTAs, more steps than a CTA's 16
+# value slots, a last block of 3, 21, 36 and 60 rows
+@pytest.mark.parametrize("nx,ny", [(1, 1), (7, 3), (13, 5), (17, 10), (19, 18)])
+@pytest.mark.parametrize("count", [1, 5, 40])
+def test_fp32_solves_with_interchanges(nx, ny, count):
+    """The cluster solves after factorisations that interchange many rows: at
+    these frequencies the off-diagonal traction terms, of order omega, exceed
+    the diagonal's 1/2.  The refinement converges only if L, its row order and
+    the block inverses agree."""
+    m = meshgen.enclosed_grid(nx, ny, jitter=0.10, seed=8, depth=2.5, layers=2)
+    d = meshgen.traction_patch(m, radius=6.0, dam=0.02)
+    d.kode[1::5] = 0
+    with BemSolver(m) as sol:
+        sol.ghmatece()
+        sol.set_bc(d.kode, d.bc, d.dam, d.rho)
+        freqs = np.linspace(12.0, 25.0, count)
+        xp, _ = sol.sweep(freqs, form="plain", batch=8)
+        xm, _ = sol.sweep(freqs, form="mixed", batch=count, refine=7)
+        for i in range(count):
+            assert rel(xm[i], xp[i]) < 1e-9, freqs[i]
