@@ -127,10 +127,12 @@ constexpr int kGroupMaps = 3;  // row maps of the first three panels of a four-p
 // Packed operands of the tensor-core FP32 trailing update (gemm_tc.cu).
 struct TcWork {
   size_t lrows_cap = 0, urows_cap = 0;  // rows the operand buffers hold
-  float* lhat = nullptr;  // [batch][2nn][64]  re/im rows of L21, TF32
+  float* lhat = nullptr;  // [batch][2nn][256] re/im rows of L21, TF32
+  float* lhat2 = nullptr;  // a second one (lookahead), made on first use
+  int lsel = 0;            // which of them is packed and multiplied now
   float* ure = nullptr;   // [batch][nn+1][64] Re U12, K-major, TF32
   float* uim = nullptr;   // [batch][nn+1][64] Im U12
-  void* maps = nullptr;   // 6 TMA tensor maps (host copies, passed by value)
+  void* maps = nullptr;   // 7 TMA tensor maps (host copies, passed by value)
   int pair_clusters = 0;  // resident CTA pairs of k_gemm_tc2 (0: not yet queried)
   float2* cbase = nullptr;  // systems the C map (maps[3]) was made for
   size_t clda = 0, cbstride = 0;
@@ -218,6 +220,11 @@ struct bem_ctx {
   int sg_nn = 0, sg_bsz = 0, sg_mixed = 0, sg_iters = 0;
   long long sg_launches = 0;
   int sw_nn = 0, sw_bsz = 0, sw_mixed = 0, sw_iters = 0;  // shape of the last directly enqueued step
+  // the critical path of a factorisation with lookahead (made on first use)
+  cudaStream_t crit = nullptr;
+  cudaEvent_t crit_ev[3] = {nullptr, nullptr, nullptr};
+  void* crit_ws = nullptr;    // cuBLAS workspace of its products
+  bool lu_lookahead = true;   // LU: panels run beside the previous group's update
   bool panel_calu = false;    // FP32 LU panels: tournament pivoting per 8-column sub-panel
   bool panel_push = true;     // cluster panels exchange pivots by remote stores before the barrier
   bool panel_async = true;    // ... as st.async into mbarrier-counted mailboxes, no per-column cluster barrier
@@ -356,12 +363,13 @@ const double2* slot_batch_solution(bem_ctx* ctx, bool mixed, int b);
 
 // Tensor-core FP32 trailing update (gemm_tc.cu).
 int tc_ensure(bem_ctx* ctx, int nn, int batch);
+int tc_ensure_second(bem_ctx* ctx);
 void tc_release(bem_ctx* ctx);
 int tc_trailing_update(bem_ctx* ctx, float2* A, size_t lda, size_t bstride, int nn, int k, int w, int batch);
 int tc_pack_l(bem_ctx* ctx, const float2* A, size_t lda, size_t bstride, int nn, int kcol, int kw, int r0, int koff,
               int batch, const int* gmap, size_t gstride, int npanels = 1, int nmaps = 1);
 int tc_gemm(bem_ctx* ctx, float2* A, size_t lda, size_t bstride, int nn, int r0, int c0, int cend, int kw,
-            int urow_off, int batch, int kbase);
+            int urow_off, int batch, int kbase, int tiles = 0);
 constexpr int kTcKPitch = 256;  // floats per packed tensor-core operand row
 
 // One 32-row block of the packed tensor-core operand Lhat (256 threads):

@@ -237,6 +237,9 @@ int bem_ctx_destroy(bem_ctx* ctx) {
   release_cublas(ctx);
   tc_release(ctx);
   for (cudaEvent_t e : ctx->prof.pool) cudaEventDestroy(e);
+  if (ctx->crit) cudaStreamDestroy(ctx->crit);
+  for (cudaEvent_t e : ctx->crit_ev)
+    if (e) cudaEventDestroy(e);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
   return BEM_OK;
@@ -611,6 +614,7 @@ static bool* option_slot(bem_ctx* ctx, const char* name) {
   if (!strcmp(name, "lu_quads")) return &ctx->lu_quads;
   if (!strcmp(name, "f64_pairs")) return &ctx->f64_pairs;
   if (!strcmp(name, "f64_cublas")) return &ctx->f64_cublas;
+  if (!strcmp(name, "lu_lookahead")) return &ctx->lu_lookahead;
   if (!strcmp(name, "tc_pair")) return &ctx->tc_pair;
   if (!strcmp(name, "small_clusters")) return &ctx->small_clusters;
   if (!strcmp(name, "panel_tslu")) return &ctx->panel_tslu;

@@ -91,6 +91,8 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, int x,
       : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+// (one group per half, so that waiting for all but one means the other half's)
+__device__ __forceinline__ void tma_commit_empty() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -139,6 +141,7 @@ struct TcArgs {
   int band;         // m-tiles per band of the tile order (see tile_of)
   int lrows;        // Lhat rows per problem (2*nn)
   int urows;        // U rows per problem (nn+1)
+  int chunk;        // k_gemm_tc2: adjacent tiles per CTA pair (0: persistent pairs)
   int* status;
 };
 
@@ -439,6 +442,9 @@ __global__ void __launch_bounds__(256, 1) k_gemm_tc2(const __grid_constant__ CUt
   const bool even = rank == 0;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int total = a.mtiles * a.ntiles * a.batch;  // mtiles: 128-complex-row tiles here
+  // this pair's tiles: every npairs-th (persistent), or a.chunk adjacent ones
+  const int t0 = a.chunk ? pair * a.chunk : pair, tstep = a.chunk ? 1 : npairs;
+  const int t1 = a.chunk ? min(total, t0 + a.chunk) : total;
   const int nchunks = (a.kw + 31) / 32;
 
   if (threadIdx.x == 0) {
@@ -472,7 +478,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_tc2(const __grid_constant__ CUt
     int s = 0;
     uint32_t ph = 0;
     bool ok = true;
-    for (int t = pair; t < total && ok; t += npairs) {
+    for (int t = t0; t < t1 && ok; t += tstep) {
       int b, tm, tn;
       tile_of(t, a, b, tm, tn);
       const int ly = b * a.lrows + 2 * (tm * tile_rows + (int)rank * kTcRows);
@@ -507,7 +513,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_tc2(const __grid_constant__ CUt
     uint32_t ph = 0;
     int it = 0;
     bool ok = true;
-    for (int t = pair; t < total && ok; t += npairs, ++it) {
+    for (int t = t0; t < t1 && ok; t += tstep, ++it) {
       const int buf = it & 1;
       if (!wait_or_abort(&t_empty[buf], ((uint32_t)(it >> 1) & 1u) ^ 1u, abort_flag, a.status, wlim)) break;
       tc_fence_after();
@@ -545,7 +551,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_tc2(const __grid_constant__ CUt
     const bool issuer = (e == 0 && lane == 0);
     const uint32_t te0 = pair_addr(&t_empty[0], 0), te1 = pair_addr(&t_empty[1], 0);
     int it = 0;
-    for (int t = pair; t < total; t += npairs, ++it) {
+    for (int t = t0; t < t1; t += tstep, ++it) {
       const int buf = it & 1;
       if (!__all_sync(0xffffffffu, wait_or_abort(&t_full[buf], (uint32_t)(it >> 1) & 1u, abort_flag, a.status, wlim)))
         break;
@@ -580,7 +586,13 @@ __global__ void __launch_bounds__(256, 1) k_gemm_tc2(const __grid_constant__ CUt
         }
         fence_proxy_async();
         epi_bar_sync();
-        if (issuer && row0 < a.nn) tma_reduce_add_3d(&tm_c, 2 * row0, a.c0 + tn * kTcCols + 64 * hc, b, ct);
+        if (issuer && row0 < a.nn) {
+          const int col = a.c0 + tn * kTcCols + 64 * hc;
+          if (col < a.cend)  // columns past cend may be another kernel's now
+            tma_reduce_add_3d(&tm_c, 2 * row0, col, b, ct);
+          else
+            tma_commit_empty();
+        }
       }
     }
     if (issuer) tma_store_wait_all();
@@ -749,8 +761,8 @@ int tc_ensure(bem_ctx* ctx, int nn, int batch) {
   BEM_CUDA(ctx, cudaMemsetAsync(W.ure, 0, urows * kKPitch * sizeof(float), ctx->stream));
   BEM_CUDA(ctx, cudaMemsetAsync(W.uim, 0, urows * kKPitch * sizeof(float), ctx->stream));
   // maps: 0 Lhat, 1-2 U_re/U_im (128-row boxes), 3 C (made per system), 4-5 U_re/U_im in
-  // the 64-row boxes of the CTA-pair kernel
-  W.maps = new CUtensorMap[6];
+  // the 64-row boxes of the CTA-pair kernel, 6 the second Lhat
+  W.maps = new CUtensorMap[7];
   CUtensorMap* maps = static_cast<CUtensorMap*>(W.maps);
   if (!make_map(&maps[0], W.lhat, lrows) || !make_map(&maps[1], W.ure, urows) || !make_map(&maps[2], W.uim, urows) ||
       !make_map(&maps[4], W.ure, urows, 64) || !make_map(&maps[5], W.uim, urows, 64))
@@ -762,9 +774,29 @@ int tc_ensure(bem_ctx* ctx, int nn, int batch) {
   return BEM_OK;
 }
 
+// The second Lhat: a panel group's while the previous group's update still
+// reads the first.
+int tc_ensure_second(bem_ctx* ctx) {
+  TcWork& W = ctx->tc;
+  if (W.lhat2) return BEM_OK;
+  const size_t bytes = W.lrows_cap * kKPitch * sizeof(float);
+  if (dev_alloc(ctx, &W.lhat2, bytes) != cudaSuccess) {
+    W.lhat2 = nullptr;
+    return fail(ctx, BEM_ERR_NOMEM, "no memory for a second Lhat");
+  }
+  if (!make_map(&static_cast<CUtensorMap*>(W.maps)[6], W.lhat2, W.lrows_cap)) {
+    dev_free(ctx, W.lhat2);
+    W.lhat2 = nullptr;
+    return fail(ctx, BEM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  }
+  BEM_CUDA(ctx, cudaMemsetAsync(W.lhat2, 0, bytes, ctx->stream));
+  return BEM_OK;
+}
+
 void tc_release(bem_ctx* ctx) {
   TcWork& W = ctx->tc;
   dev_free(ctx, W.lhat);
+  dev_free(ctx, W.lhat2);
   dev_free(ctx, W.ure);
   dev_free(ctx, W.uim);
   delete[] static_cast<CUtensorMap*>(W.maps);
@@ -780,7 +812,7 @@ int tc_pack_l(bem_ctx* ctx, const float2* A, size_t lda, size_t bstride, int nn,
               int batch, const int* gmap, size_t gstride, int npanels, int nmaps) {
   if (r0 >= nn) return BEM_OK;
   k_pack_l21<<<dim3((nn - r0 + 31) / 32, batch, npanels), 256, 0, ctx->stream>>>(
-      A, lda, bstride, nn, kcol, kw, r0, koff, ctx->tc.lhat, 2 * nn, gmap, gstride, gmap ? nmaps : 0);
+      A, lda, bstride, nn, kcol, kw, r0, koff, ctx->tc.lsel ? ctx->tc.lhat2 : ctx->tc.lhat, 2 * nn, gmap, gstride, gmap ? nmaps : 0);
   ctx->launches++;
   BEM_CUDA(ctx, cudaGetLastError());
   return BEM_OK;
@@ -788,8 +820,10 @@ int tc_pack_l(bem_ctx* ctx, const float2* A, size_t lda, size_t bstride, int nn,
 
 // C -= Lhat U for rows [r0, nn) and columns [c0, cend) of `batch` FP32
 // systems, K = kw (packed Lhat and U_re/U_im; U row urow_off + (c - c0)).
+// tiles > 0: at most that many per CTA pair, so that the pairs end and give
+// way to kernels of a higher priority (else persistent pairs).
 int tc_gemm(bem_ctx* ctx, float2* A, size_t lda, size_t bstride, int nn, int r0, int c0, int cend, int kw,
-            int urow_off, int batch, int kbase) {
+            int urow_off, int batch, int kbase, int tiles) {
   TcWork& W = ctx->tc;
   const int ncols = nn + 1;
   if (r0 >= nn || c0 >= cend) return BEM_OK;
@@ -846,7 +880,11 @@ int tc_gemm(bem_ctx* ctx, float2* A, size_t lda, size_t bstride, int nn, int r0,
       }
       W.pair_clusters = n;
     }
-    const int pairs = std::max(1, std::min({total, W.pair_clusters, ctas / 2}));
+    int pairs = std::max(1, std::min({total, W.pair_clusters, ctas / 2}));
+    if (tiles > 0 && total > tiles * pairs) {
+      t.chunk = tiles;
+      pairs = (total + tiles - 1) / tiles;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs, 1, 1);
     cfg.blockDim = dim3(256, 1, 1);
@@ -859,13 +897,13 @@ int tc_gemm(bem_ctx* ctx, float2* A, size_t lda, size_t bstride, int nn, int r0,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    BEM_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_gemm_tc2, maps[0], maps[4], maps[5], maps[3], t));
+    BEM_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_gemm_tc2, maps[W.lsel ? 6 : 0], maps[4], maps[5], maps[3], t));
     ctx->launches++;
     return BEM_OK;
   }
   const int total = t.mtiles * t.ntiles * batch;
   const int grid = std::min(total, ctas);
-  k_gemm_tc<<<grid, 256, kTcSmem, ctx->stream>>>(maps[0], maps[1], maps[2], maps[3], t);
+  k_gemm_tc<<<grid, 256, kTcSmem, ctx->stream>>>(maps[W.lsel ? 6 : 0], maps[1], maps[2], maps[3], t);
   ctx->launches++;
   BEM_CUDA(ctx, cudaGetLastError());
   return BEM_OK;

@@ -3892,22 +3892,31 @@ static int lockstep_capacity_t(bem_ctx* ctx, int nn) {
 // ZGEMM (the plain library GEMM, FP64 tensor cores).  L is A's columns
 // kcol..kcol+kw-1 at rows r0.., or `lg` (ld nn - r0, lg_stride per problem);
 // U is A's rows kcol..kcol+kw-1 at columns c0...  The handle and a fixed
-// workspace are made once per context, so a captured graph allocates nothing.
+// workspace are made once per context, so a captured graph allocates nothing
+// (with lookahead one more workspace: the two streams' products overlap).
 constexpr size_t kCublasWorkspace = (size_t)32 << 20;
 
-int f64_gemm_cublas(bem_ctx* ctx, double2* A, size_t lda, size_t bstride, int nn, int kcol, int kw, int r0, int c0,
-                    int cend, int batch, const double2* lg, size_t lg_stride) {
+static int ensure_cublas(bem_ctx* ctx) {
   if (!ctx->cublas) {
     cublasHandle_t h = nullptr;
     if (cublasCreate(&h) != CUBLAS_STATUS_SUCCESS) return fail(ctx, BEM_ERR_CUDA, "cublasCreate failed");
     ctx->cublas = h;
     BEM_CUDA(ctx, dev_alloc(ctx, reinterpret_cast<unsigned char**>(&ctx->cublas_ws), kCublasWorkspace));
     BEM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (cublasSetWorkspace(h, ctx->cublas_ws, kCublasWorkspace) != CUBLAS_STATUS_SUCCESS)
-      return fail(ctx, BEM_ERR_CUDA, "cublasSetWorkspace failed");
   }
+  return BEM_OK;
+}
+
+int f64_gemm_cublas(bem_ctx* ctx, double2* A, size_t lda, size_t bstride, int nn, int kcol, int kw, int r0, int c0,
+                    int cend, int batch, const double2* lg, size_t lg_stride) {
+  int rc = ensure_cublas(ctx);
+  if (rc) return rc;
   cublasHandle_t h = static_cast<cublasHandle_t>(ctx->cublas);
+  // setting the stream also resets the workspace
   if (cublasSetStream(h, ctx->stream) != CUBLAS_STATUS_SUCCESS) return fail(ctx, BEM_ERR_CUDA, "cublasSetStream failed");
+  if (cublasSetWorkspace(h, ctx->stream == ctx->crit ? ctx->crit_ws : ctx->cublas_ws, kCublasWorkspace) !=
+      CUBLAS_STATUS_SUCCESS)
+    return fail(ctx, BEM_ERR_CUDA, "cublasSetWorkspace failed");
   const int m = nn - r0, n = cend - c0;
   if (m <= 0 || n <= 0 || kw <= 0) return BEM_OK;
   const cuDoubleComplex minus_one = make_cuDoubleComplex(-1.0, 0.0), one = make_cuDoubleComplex(1.0, 0.0);
@@ -3921,11 +3930,6 @@ int f64_gemm_cublas(bem_ctx* ctx, double2* A, size_t lda, size_t bstride, int nn
   if (st != CUBLAS_STATUS_SUCCESS) return fail(ctx, BEM_ERR_CUDA, "cublasZgemmStridedBatched failed");
   ctx->launches++;
   return BEM_OK;
-}
-
-int f64_update_cublas(bem_ctx* ctx, double2* A, size_t lda, size_t bstride, int nn, int k, int w, int c0, int ncols,
-                      int batch) {
-  return f64_gemm_cublas(ctx, A, lda, bstride, nn, k, w, c0, c0, ncols, batch, nullptr, 0);
 }
 
 // L of an FP64 panel pair for its update past the pair (rows r0.. of columns
@@ -3976,6 +3980,8 @@ void release_cublas(bem_ctx* ctx) {
   ctx->cublas = nullptr;
   dev_free(ctx, ctx->cublas_ws);
   ctx->cublas_ws = nullptr;
+  dev_free(ctx, ctx->crit_ws);
+  ctx->crit_ws = nullptr;
 }
 
 // Problems whose panels run in one wave: the first (tallest) panel's cluster
@@ -4339,6 +4345,120 @@ static int trsv_coop(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, in
   return BEM_OK;
 }
 
+// Lookahead of the factorisation: panels, and what the next panels need, run
+// on a stream of the highest priority (ctx->crit) while the context's stream
+// applies the last group's update to the columns past the next group.  A
+// panel keeps 1..16 SMs per problem busy, so one after the other left most of
+// the device idle for a third of the time; with priorities the update's CTAs
+// give way as they end (FP64, 6480 unknowns: four panels of 191 us beside a
+// trailing update of 1300 us took 1392 us, and the panels 200 us each;
+// without priorities the panels waited for the update's end).
+// Group g with columns [k, kG), the next group's [kG, kN):
+//   crit:  the group's panels and their updates inside the group; then, once
+//          the main stream has finished group g - 1 (crit_waits), the
+//          last interchanges, the packing of L (record_pack) and the update
+//          of [kG, kN).
+//   main:  each panel's interchanges of [kG, ncols) as it is done
+//          (main_waits), the last one's of [kN, ncols) only; the update of
+//          [kN, ncols).
+// Every column takes the same operations in the same order as without it.
+struct Lookahead {
+  bem_ctx* ctx;
+  cudaStream_t main;
+  bool on = false;
+  explicit Lookahead(bem_ctx* c) : ctx(c), main(c->stream) {}
+  Lookahead(const Lookahead&) = delete;
+  ~Lookahead() { join(); }  // also after an error: nothing of crit outlives the call
+  int order(cudaStream_t before, cudaEvent_t ev, cudaStream_t after) {
+    BEM_CUDA(ctx, cudaEventRecord(ev, before));
+    BEM_CUDA(ctx, cudaStreamWaitEvent(after, ev, 0));
+    return BEM_OK;
+  }
+  int fork() {
+    if (!ctx->crit) {
+      int lo = 0, hi = 0;
+      BEM_CUDA(ctx, cudaDeviceGetStreamPriorityRange(&lo, &hi));
+      for (cudaEvent_t& e : ctx->crit_ev)
+        if (!e) BEM_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      BEM_CUDA(ctx, cudaStreamCreateWithPriority(&ctx->crit, cudaStreamNonBlocking, hi));
+    }
+    int rc = order(main, ctx->crit_ev[0], ctx->crit);
+    if (rc) return rc;
+    on = true;
+    use_crit();
+    return BEM_OK;
+  }
+  int join() {
+    if (!on) return BEM_OK;
+    on = false;
+    use_main();
+    return order(ctx->crit, ctx->crit_ev[1], main);
+  }
+  void use_crit() { ctx->stream = ctx->crit; }
+  void use_main() { ctx->stream = main; }
+  int main_waits() { return order(ctx->crit, ctx->crit_ev[1], main); }
+  int crit_waits() { return order(main, ctx->crit_ev[0], ctx->crit); }
+  int record_pack() {
+    BEM_CUDA(ctx, cudaEventRecord(ctx->crit_ev[2], ctx->crit));
+    return BEM_OK;
+  }
+  int main_waits_pack() {
+    BEM_CUDA(ctx, cudaStreamWaitEvent(main, ctx->crit_ev[2], 0));
+    return BEM_OK;
+  }
+};
+
+// Tiles per CTA pair of an update beside panels: it then ends often enough
+// for a panel's cluster to find its SMs (25920 unknowns: 167 ms with 2, 152
+// with 4 and 8, 156 with 16, 162 with 32; persistent pairs 185, no gain).
+constexpr int kLookTiles = 8;
+
+// Is lookahead worth its launches?  All panels have to be resident at once,
+// and an update has to take a panel's time: nn^2 batch above 2.5e6 in FP64
+// (ms off / on: 1530 x 1: 3.37 / 3.43, x 4: 4.43 / 3.95; 1800 x 9: 8.84 /
+// 7.76; 3240 x 1: 10.3 / 8.5; 6480 x 1: 40.1 / 30.9), above 2.5e7 in FP32
+// (1530 x 8: 3.36 / 3.37; 2871 x 4: 6.65 / 6.47, x 10: 8.29 / 7.78; 6480 x 10:
+// 36.0 / 32.5; 25920 x 1: 185 / 151).  nn > 256: at least one group.
+template <typename R>
+static bool lookahead_shape(bem_ctx* ctx, int nn, int batch) {
+  const double work = (double)nn * nn * batch;
+  if (nn <= 256 || work < (sizeof(R) == 8 ? 2.5e6 : 2.5e7)) return false;
+  const PanelShape sh = panel_shape<R>(ctx, nn, batch);
+  return sh.cs > 0 && sh.cs * batch <= ctx->num_sms;
+}
+
+// Is there memory for `bytes` more with as much again, several times, left for
+// the solves' buffers?  (Lookahead may not take what a call needs without it.)
+static bool lookahead_room(bem_ctx* ctx, size_t bytes) {
+  size_t avail = 0, total = 0;
+  unsigned long long reserved = 0, used = 0;
+  cudaMemPool_t pool;
+  if (cudaMemGetInfo(&avail, &total) != cudaSuccess || cudaDeviceGetDefaultMemPool(&pool, ctx->device) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return false;
+  return avail + (size_t)(reserved - used) > 4 * bytes + ((size_t)1 << 30);
+}
+
+// What the two streams of an FP64 factorisation need: a workspace each and the
+// first (largest) pair's L.
+static size_t lookahead_lg(int nn, int batch) { return (size_t)(nn - 128) * 128 * batch; }
+static int lookahead_f64_buffers(bem_ctx* ctx, int nn, int batch) {
+  int rc = ensure_cublas(ctx);
+  if (rc) return rc;
+  if (!ctx->crit_ws) BEM_CUDA(ctx, dev_alloc(ctx, reinterpret_cast<unsigned char**>(&ctx->crit_ws), kCublasWorkspace));
+  LuWork& LW = ctx->lu;
+  const size_t need = lookahead_lg(nn, batch);
+  if (LW.lg_cap < need) {
+    dev_free(ctx, LW.lg);
+    LW.lg = nullptr;
+    LW.lg_cap = 0;
+    BEM_CUDA(ctx, dev_alloc(ctx, &LW.lg, need * sizeof(double2)));
+    LW.lg_cap = need;
+  }
+  return BEM_OK;
+}
+
 template <typename R>
 static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int batch) {
   LuWork& L = ctx->lu;
@@ -4453,9 +4573,10 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
   };
   // L11^-1 of the panel at k (for k_laswp_tc) and, for panel gi of a group
   // of gsize, the group's row maps (k_l11_inv).
-  auto linv_maps = [&](int k, int w, const int* perm_p, int gi, int gsize) -> int {
+  const size_t linv_slot = (size_t)batch * kLfragMats * kLfragMat;
+  auto linv_ensure = [&](int slots) -> int {
     LuWork& LW = ctx->lu;
-    const size_t lbytes = (size_t)batch * kLfragMats * kLfragMat * sizeof(float);
+    const size_t lbytes = slots * linv_slot * sizeof(float);
     if (LW.linv_bytes < lbytes) {
       dev_free(ctx, LW.linv);
       LW.linv = nullptr;
@@ -4471,24 +4592,32 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
       BEM_CUDA(ctx, dev_alloc(ctx, &LW.gmap, mbytes));
       LW.gmap_bytes = mbytes;
     }
+    return BEM_OK;
+  };
+  auto linv_maps = [&](int k, int w, const int* perm_p, int gi, int gsize, int slot) -> int {
+    int rc = linv_ensure(slot + 1);
+    if (rc) return rc;
     BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_l11_inv), (2 * kLtTile)));
     k_l11_inv<<<dim3(1 + std::min(std::max(gi, 0), kGroupMaps), batch), 1024, 2 * kLtTile, ctx->stream>>>(
-        static_cast<const float2*>(A), lda, bstride, k, w, LW.linv, perm_p, kPermStride, LW.gmap, nn, gi, gsize);
+        static_cast<const float2*>(A), lda, bstride, k, w, ctx->lu.linv + slot * linv_slot, perm_p, kPermStride,
+        ctx->lu.gmap, nn, gi, gsize);
     ctx->launches++;
     BEM_CUDA(ctx, cudaGetLastError());
     return BEM_OK;
   };
-  // Interchanges + U12 of the panel at k for columns [c0, ncols), packed for
+  // Interchanges + U12 of the panel at k for columns [c0, cend), packed for
   // the tensor cores at K slot koff (rows c - ubase).  Columns from cdefer
   // on first take the deferred update of the nprev earlier panels of the
   // group (at kfirst, kfirst + 64, ...); gi/gsize: the panel's place in its
   // group (-1: none).
   // pack_r0 >= 0: also pack this panel's L21 (rows pack_r0..) at K slot koff
   // for the update that follows (packed = true when done here).
-  auto laswp = [&](int k, int w, int c0, const int* perm_p, int ubase, int koff, int kfirst, int nprev, int cdefer,
-                   int gi, int gsize, int pack_r0, bool& packed) -> int {
+  // slot: where L11^-1 is kept; have_linv: linv_maps of this panel is done.
+  auto laswp = [&](int k, int w, int c0, int cend, const int* perm_p, int ubase, int koff, int kfirst, int nprev,
+                   int cdefer, int gi, int gsize, int pack_r0, bool& packed, int slot = 0,
+                   bool have_linv = false) -> int {
     packed = false;
-    const int cols = ncols - c0;
+    const int cols = cend - c0;
     if (cols <= 0) return BEM_OK;
     const bool pre = nprev > 0;
     // rows k..k+w-1 (and the displaced rows) of every column read and written once
@@ -4496,27 +4625,31 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     float* ure = tc ? ctx->tc.ure : nullptr;
     float* uim = tc ? ctx->tc.uim : nullptr;
     if (sizeof(R) == 4 && ctx->laswp_tc) {
-      int rc = linv_maps(k, w, perm_p, gi, gsize);
-      if (rc) return rc;
+      if (!have_linv) {
+        int rc = linv_maps(k, w, perm_p, gi, gsize, slot);
+        if (rc) return rc;
+      }
+      const float* const linv = ctx->lu.linv + slot * linv_slot;
       // two CTAs per SM
       const int ntiles = (cols + kLtCols - 1) / kLtCols;
       const int per = std::max(1, 2 * ctx->num_sms / batch);
-      const int tb = std::min(ntiles, per);
+      const int pk = (ure && pack_r0 >= 0) ? pack_r0 : -1;
+      // the packing's 32-row blocks may ask for more CTAs than the tiles do
+      // (a group's 192 columns alone: 6 CTAs packed 25920 rows in 260 us)
+      const int tb = std::min(std::max(ntiles, pk >= 0 ? (nn - pk + 63) / 64 : 0), per);
       const size_t sm = (1 + nprev) * kLtColTile;
       float2* A2 = static_cast<float2*>(A);
-      LuWork& LW = ctx->lu;
-      const int pk = (ure && pack_r0 >= 0) ? pack_r0 : -1;
-      float* lhat = ctx->tc.lhat;
+      float* lhat = ctx->tc.lsel ? ctx->tc.lhat2 : ctx->tc.lhat;
       if (pre) {
         BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_tc<true>), sm));
         k_laswp_tc<true><<<dim3(tb, batch), 256, sm, ctx->stream>>>(
-            A2, lda, bstride, k, w, c0, ncols, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, nprev,
-            cdefer, nn, LW.linv, lhat, 2 * nn, pk);
+            A2, lda, bstride, k, w, c0, cend, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, nprev,
+            cdefer, nn, linv, lhat, 2 * nn, pk);
       } else {
         BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_laswp_tc<false>), sm));
         k_laswp_tc<false><<<dim3(tb, batch), 256, sm, ctx->stream>>>(
-            A2, lda, bstride, k, w, c0, ncols, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, 0, ncols, nn,
-            LW.linv, lhat, 2 * nn, pk);
+            A2, lda, bstride, k, w, c0, cend, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, 0, cend, nn,
+            linv, lhat, 2 * nn, pk);
       }
       ctx->launches++;
       BEM_CUDA(ctx, cudaGetLastError());
@@ -4524,7 +4657,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
       return BEM_OK;
     }
     if (gi >= 0 && sizeof(R) == 4) {  // the grouped packs read L through the row maps
-      int rc = linv_maps(k, w, perm_p, gi, gsize);
+      int rc = linv_maps(k, w, perm_p, gi, gsize, 0);
       if (rc) return rc;
     }
     if constexpr (sizeof(R) == 8) {
@@ -4534,7 +4667,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
       const int per = std::max(1, ctx->num_sms / batch), nt8 = (cols + 7) / 8;
       auto launch = [&](auto kern, size_t sm, int tiles) -> int {
         BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(kern), sm));
-        kern<<<dim3(std::min(tiles, per), batch), 256, sm, ctx->stream>>>(A2, lda, bstride, k, w, c0, ncols, perm_p,
+        kern<<<dim3(std::min(tiles, per), batch), 256, sm, ctx->stream>>>(A2, lda, bstride, k, w, c0, cend, perm_p,
                                                                           kPermStride, kfirst, k - kfirst);
         ctx->launches++;
         BEM_CUDA(ctx, cudaGetLastError());
@@ -4550,15 +4683,89 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     const int blocks = std::max(1, std::min((cols + 31) / 32, (4 * ctx->num_sms + batch - 1) / batch));
     if (pre)
       k_laswp_trsm<R, true><<<dim3(blocks, batch), 256, 2 * lsmem, ctx->stream>>>(
-          A, lda, bstride, k, w, c0, ncols, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, k - kfirst);
+          A, lda, bstride, k, w, c0, cend, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, k - kfirst);
     else
       k_laswp_trsm<R, false><<<dim3(blocks, batch), 256, lsmem, ctx->stream>>>(
-          A, lda, bstride, k, w, c0, ncols, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, 0);
+          A, lda, bstride, k, w, c0, cend, perm_p, kPermStride, ure, uim, nn + 1, ubase, koff, kfirst, 0);
     ctx->launches++;
     BEM_CUDA(ctx, cudaGetLastError());
     return BEM_OK;
     }
   };
+  // FP64 updates of columns [c0, cend): one panel's of rows r0.., and a pair's
+  // of the rows past the pair.
+  auto f64_one = [&](int k, int w, int r0, int c0, int cend) -> int {
+    double2* A2 = static_cast<double2*>(A);
+    if (ctx->f64_cublas) return f64_gemm_cublas(ctx, A2, lda, bstride, nn, k, w, r0, c0, cend, batch, nullptr, 0);
+    dim3 grid((nn - r0 + GBM - 1) / GBM, (cend - c0 + GBN - 1) / GBN, batch);
+    k_gemm_f64<<<grid, 256, kGemmSmem, ctx->stream>>>(A2, lda, bstride, nn, k, w, r0, c0, cend, nullptr, 0, 0);
+    ctx->launches++;
+    BEM_CUDA(ctx, cudaGetLastError());
+    return BEM_OK;
+  };
+  // both panels' L in one buffer (the first through the second's gather list)
+  auto f64_gather = [&](int k, int w1, int w2, const int* p2) -> int {
+    LuWork& LW = ctx->lu;
+    const int kG = k + w1 + w2;
+    const size_t per = (size_t)(nn - kG) * (w1 + w2), need = per * batch;
+    if (LW.lg_cap < need) {
+      dev_free(ctx, LW.lg);
+      LW.lg = nullptr;
+      LW.lg_cap = 0;
+      BEM_CUDA(ctx, dev_alloc(ctx, &LW.lg, need * sizeof(double2)));
+      LW.lg_cap = need;
+    }
+    k_gather_l_pair<<<dim3((nn - kG + 255) / 256, (w1 + w2 + kGatherCols - 1) / kGatherCols, batch), 256, 0,
+                      ctx->stream>>>(static_cast<const double2*>(A), lda, bstride, nn, k, w1, w2, kG, p2, kPermStride,
+                                     LW.lg, per);
+    ctx->launches++;
+    BEM_CUDA(ctx, cudaGetLastError());
+    return BEM_OK;
+  };
+  auto f64_pair = [&](int k, int w1, int w2, const int* p2, int c0, int cend) -> int {
+    const int kG = k + w1 + w2;
+    double2* A2 = static_cast<double2*>(A);
+    if (ctx->f64_cublas)
+      return f64_gemm_cublas(ctx, A2, lda, bstride, nn, k, w1 + w2, kG, c0, cend, batch, ctx->lu.lg,
+                             (size_t)(nn - kG) * (w1 + w2));
+    dim3 grid((nn - kG + GBM - 1) / GBM, (cend - c0 + GBN - 1) / GBN, batch);
+    k_gemm_f64<<<grid, 256, kGemmSmem, ctx->stream>>>(A2, lda, bstride, nn, k, w1 + w2, kG, c0, cend, p2, kPermStride,
+                                                     w1);
+    ctx->launches++;
+    BEM_CUDA(ctx, cudaGetLastError());
+    return BEM_OK;
+  };
+  // Lookahead: the default kernels only, and not while kernel classes are
+  // timed one by one or the context has only a share of the SMs.
+  bool look = ctx->lu_lookahead && !ctx->prof.on && ctx->gemm_ctas == 0 && ip &&
+                    (sizeof(R) == 8 ? ctx->f64_pairs && ctx->f64_cublas
+                                    : tc && ctx->tc_pair && ctx->lu_quads && ctx->lu_pairs && ctx->laswp_tc) &&
+                    lookahead_shape<R>(ctx, nn, batch);
+  Lookahead la(ctx);
+  int gpar = 0;  // parity of the group: its packed L and L11^-1 while the previous group's are in use
+  ctx->tc.lsel = 0;
+  if (look) {
+    // the two streams' buffers, before they part; without the memory for them
+    // (and in a capture, which must not allocate) one stream does
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    BEM_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+      look = ctx->crit && (sizeof(R) == 4 ? L.linv_bytes >= 8 * linv_slot * sizeof(float) &&
+                                                L.gmap_bytes >= (size_t)batch * kGroupMaps * nn * sizeof(int) &&
+                                                ctx->tc.lhat2
+                                          : ctx->cublas && ctx->crit_ws && L.lg_cap >= lookahead_lg(nn, batch));
+    else
+      look = sizeof(R) == 4
+                 ? (ctx->tc.lhat2 || lookahead_room(ctx, ctx->tc.lrows_cap * kTcKPitch * sizeof(float))) &&
+                       linv_ensure(8) == BEM_OK && tc_ensure_second(ctx) == BEM_OK
+                 : (ctx->crit_ws || lookahead_room(ctx, kCublasWorkspace)) &&
+                       lookahead_f64_buffers(ctx, nn, batch) == BEM_OK;
+    cudaGetLastError();
+  }
+  if (look) {
+    int rc = la.fork();
+    if (rc) return rc;
+  }
   for (int k = 0; k < nn;) {
     const int m = nn - k;
     // G = 2 or 4 64-column panels per trailing update (K = 64 G) on the
@@ -4582,6 +4789,49 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     const bool fit4 = m > 256 && pw(m) == 64 && pw(m - 64) == 64 && pw(m - 128) == 64 && pw(m - 192) == 64;
     const bool fit2 = m > 128 && pw(m) == 64 && pw(m - 64) == 64;
     const int G = (tcg && ctx->lu_quads && ctx->laswp_tc && fit4) ? 4 : ((tcg && ctx->lu_pairs && fit2) ? 2 : 1);
+    if (G > 1 && look) {
+      const int kG = k + 64 * G, kN = std::min(kG + 256, ncols);
+      float2* A2 = static_cast<float2*>(A);
+      ctx->tc.lsel = gpar;
+      bool packed = false;
+      for (int i = 0; i < G; ++i) {
+        const int ki = k + 64 * i, slot = 4 * gpar + i, r0 = ki + 64;
+        int wi = 0, *pi = nullptr;
+        int rc = run_panel(ki, wi, pi);
+        if (!rc) rc = linv_maps(ki, 64, pi, i, G, slot);
+        if (!rc) rc = la.main_waits();
+        if (rc) return rc;
+        if (i < G - 1) {
+          rc = laswp(ki, 64, r0, kG, pi, 0, 64 * i, k, i, kG, i, G, r0, packed, slot, true);
+          if (!rc) rc = tc_gemm(ctx, A2, lda, bstride, nn, r0, r0, kG, 64, r0, batch, 64 * i);
+          if (rc) return rc;
+          la.use_main();
+          rc = laswp(ki, 64, kG, ncols, pi, 0, 64 * i, k, i, kG, i, G, -1, packed, slot, true);
+          la.use_crit();
+          if (rc) return rc;
+          continue;
+        }
+        rc = la.crit_waits();
+        if (!rc) rc = laswp(ki, 64, kG, kN, pi, 0, 64 * i, k, i, kG, i, G, -1, packed, slot, true);
+        if (!rc)
+          rc = tc_pack_l(ctx, A2, lda, bstride, nn, k, 64, kG, 0, batch, ctx->lu.gmap, (size_t)kGroupMaps * nn, G,
+                         G - 1);
+        if (!rc) rc = la.record_pack();
+        if (!rc) rc = tc_gemm(ctx, A2, lda, bstride, nn, kG, kG, kN, 64 * G, kG, batch, 0);
+        if (rc) return rc;
+        if (kN < ncols) {
+          la.use_main();
+          rc = laswp(ki, 64, kN, ncols, pi, 0, 64 * i, k, i, kG, i, G, -1, packed, slot, true);
+          if (!rc) rc = la.main_waits_pack();
+          if (!rc) rc = tc_gemm(ctx, A2, lda, bstride, nn, kG, kN, ncols, 64 * G, kN, batch, 0, kLookTiles);
+          la.use_crit();
+          if (rc) return rc;
+        }
+      }
+      gpar ^= 1;
+      k = kG;
+      continue;
+    }
     if (G > 1) {
       const int kG = k + 64 * G, ubase = k + 64;
       float2* A2 = static_cast<float2*>(A);
@@ -4591,7 +4841,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
         int rc = run_panel(ki, wi, pi);
         if (rc) return rc;
         bool packed = false;
-        rc = laswp(ki, 64, ki + 64, pi, ubase, 64 * i, k, i, kG, i, G, i < G - 1 ? ki + 64 : -1, packed);
+        rc = laswp(ki, 64, ki + 64, ncols, pi, ubase, 64 * i, k, i, kG, i, G, i < G - 1 ? ki + 64 : -1, packed);
         if (rc) return rc;
         if (i < G - 1) {  // panel i's update of the group's remaining columns
           const int r0 = ki + 64;
@@ -4617,73 +4867,61 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     // FP64: two panels of the same width nb per trailing update (K = 2 nb).
     // Panel 1's update reaches panel 2's columns at once (a narrow update);
     // past the pair, panel 2's interchanges reach rows that have not taken
-    // panel 1's update, panel 2's U rows first take it (k_laswp_trsm<PRE>,
+    // panel 1's update, panel 2's U rows first take it (k_laswp_f64<PRE>,
     // panel 1's L read at panel 2's rows through its gather list), and the
     // rest is one K = 2 nb update whose first nb columns read panel 1's L
     // through the same list.  A keeps the factors of the one-panel-at-a-time
     // LU, so the solves are unchanged.
     const int nbp = sizeof(R) == 8 && ctx->f64_pairs ? panel_nb(m) : 0;
     if (nbp > 0 && m > 2 * nbp && panel_nb(m - nbp) == nbp) {
-      double2* A2 = static_cast<double2*>(A);
       int w1 = 0, w2 = 0, *p1 = nullptr, *p2 = nullptr;
-      int rc = run_panel(k, w1, p1);
-      if (rc) return rc;
-      const int k2 = k + w1;
+      const int k2 = k + nbp, kG = k2 + nbp, kN = look ? std::min(kG + 128, ncols) : ncols;
       bool packed = false;
-      rc = laswp(k, w1, k2, p1, k2, 0, k, 0, k2, -1, 1, -1, packed);
+      int rc = run_panel(k, w1, p1);
+      if (!rc && look) rc = la.main_waits();
+      if (!rc) rc = laswp(k, w1, k2, look ? kG : ncols, p1, k2, 0, k, 0, k2, -1, 1, -1, packed);
       if (rc) return rc;
       {  // panel 1's update of panel 2's columns
         ProfScope ps(ctx, 3, 8.0 * (double)(nn - k2) * (double)nbp * (double)w1 * batch,
                      2.0 * (double)(nn - k2) * (double)nbp * es * batch);
-        if (ctx->f64_cublas) {
-          rc = f64_gemm_cublas(ctx, A2, lda, bstride, nn, k, w1, k2, k2, k2 + nbp, batch, nullptr, 0);
-          if (rc) return rc;
-        } else {
-          dim3 grid((nn - k2 + GBM - 1) / GBM, (nbp + GBN - 1) / GBN, batch);
-          k_gemm_f64<<<grid, 256, kGemmSmem, ctx->stream>>>(A2, lda, bstride, nn, k, w1, k2, k2, k2 + nbp, nullptr,
-                                                           0, 0);
-          ctx->launches++;
-          BEM_CUDA(ctx, cudaGetLastError());
-        }
+        rc = f64_one(k, w1, k2, k2, kG);
+        if (rc) return rc;
       }
       rc = run_panel(k2, w2, p2);
       if (rc) return rc;
-      const int kG = k2 + w2;
-      rc = laswp(k2, w2, kG, p2, kG, 0, k, 1, kG, -1, 1, -1, packed);
+      if (look) {
+        la.use_main();
+        rc = laswp(k, w1, kG, ncols, p1, k2, 0, k, 0, k2, -1, 1, -1, packed);
+        la.use_crit();
+        if (!rc) rc = la.crit_waits();
+        if (!rc) rc = la.main_waits();
+        if (rc) return rc;
+      }
+      rc = laswp(k2, w2, kG, kN, p2, kG, 0, k, 1, kG, -1, 1, -1, packed);
       if (rc) return rc;
       if (kG < nn) {
-        const int cols = ncols - kG;
-        ProfScope ps(ctx, 3, 8.0 * (double)(nn - kG) * (double)cols * (double)(w1 + w2) * batch,
-                     2.0 * (double)(nn - kG) * (double)cols * es * batch);
-        if (ctx->f64_cublas) {
-          // both panels' L in one buffer (the first through the second's
-          // gather list), then one ZGEMM with K = w1 + w2
-          LuWork& LW = ctx->lu;
-          const size_t per = (size_t)(nn - kG) * (w1 + w2), need = per * batch;
-          if (LW.lg_cap < need) {
-            dev_free(ctx, LW.lg);
-            LW.lg = nullptr;
-            LW.lg_cap = 0;
-            BEM_CUDA(ctx, dev_alloc(ctx, &LW.lg, need * sizeof(double2)));
-            LW.lg_cap = need;
-          }
-          k_gather_l_pair<<<dim3((nn - kG + 255) / 256, (w1 + w2 + kGatherCols - 1) / kGatherCols, batch), 256, 0,
-                            ctx->stream>>>(
-              A2, lda, bstride, nn, k, w1, w2, kG, p2, kPermStride, LW.lg, per);
-          ctx->launches++;
-          BEM_CUDA(ctx, cudaGetLastError());
-          rc = f64_gemm_cublas(ctx, A2, lda, bstride, nn, k, w1 + w2, kG, kG, ncols, batch, LW.lg, per);
+        ProfScope ps(ctx, 3, 8.0 * (double)(nn - kG) * (double)(ncols - kG) * (double)(w1 + w2) * batch,
+                     2.0 * (double)(nn - kG) * (double)(ncols - kG) * es * batch);
+        if (ctx->f64_cublas) rc = f64_gather(k, w1, w2, p2);
+        if (!rc && kN < ncols) rc = la.record_pack();
+        if (!rc) rc = f64_pair(k, w1, w2, p2, kG, kN);
+        if (rc) return rc;
+        if (kN < ncols) {
+          la.use_main();
+          rc = laswp(k2, w2, kN, ncols, p2, kG, 0, k, 1, kG, -1, 1, -1, packed);
+          if (!rc) rc = la.main_waits_pack();
+          if (!rc) rc = f64_pair(k, w1, w2, p2, kN, ncols);
+          la.use_crit();
           if (rc) return rc;
-        } else {
-          dim3 grid((nn - kG + GBM - 1) / GBM, (cols + GBN - 1) / GBN, batch);
-          k_gemm_f64<<<grid, 256, kGemmSmem, ctx->stream>>>(A2, lda, bstride, nn, k, w1 + w2, kG, kG, ncols, p2,
-                                                           kPermStride, w1);
-          ctx->launches++;
-          BEM_CUDA(ctx, cudaGetLastError());
         }
       }
       k = kG;
       continue;
+    }
+    if (look) {  // a panel by itself: its update of every column on the critical stream
+      int rcw = la.crit_waits();
+      if (rcw) return rcw;
+      ctx->tc.lsel = 0;
     }
     int w = 0, *perm_p = nullptr;
     int rc = run_panel(k, w, perm_p);
@@ -4692,7 +4930,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     if (c0 < ncols) {
       const int cols = ncols - c0;
       bool packed = false;
-      rc = laswp(k, w, c0, perm_p, c0, 0, k, 0, c0, -1, 1, tc ? c0 : -1, packed);
+      rc = laswp(k, w, c0, ncols, perm_p, c0, 0, k, 0, c0, -1, 1, tc ? c0 : -1, packed);
       if (rc) return rc;
       if (c0 < nn) {
         ProfScope ps(ctx, 3, 8.0 * (double)(nn - c0) * (double)cols * (double)w * batch,
@@ -4703,14 +4941,9 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
           else
             rc = tc_trailing_update(ctx, static_cast<float2*>(A), lda, bstride, nn, k, w, batch);
           if (rc) return rc;
-        } else if (sizeof(R) == 8 && ctx->f64_cublas) {
-          rc = f64_update_cublas(ctx, static_cast<double2*>(A), lda, bstride, nn, k, w, c0, ncols, batch);
-          if (rc) return rc;
         } else if (sizeof(R) == 8) {
-          dim3 grid((nn - c0 + GBM - 1) / GBM, (cols + GBN - 1) / GBN, batch);
-          k_gemm_f64<<<grid, 256, kGemmSmem, ctx->stream>>>(static_cast<double2*>(A), lda, bstride, nn, k, w, c0, c0,
-                                                           ncols, nullptr, 0, 0);
-          ctx->launches++;
+          rc = f64_one(k, w, c0, c0, ncols);
+          if (rc) return rc;
         } else {
           dim3 grid((nn - c0 + TBM - 1) / TBM, (cols + TBN - 1) / TBN, batch);
           k_gemm_tf32<<<grid, 256, kGemmTf32Smem, ctx->stream>>>(static_cast<float2*>(A), lda, bstride, nn, k, w, c0,
@@ -4721,6 +4954,10 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
       }
     }
     k += w;
+  }
+  {
+    int rc = la.join();
+    if (rc) return rc;
   }
   ProfScope ps(ctx, 4, 4.0 * (double)nn * nn * batch, 0.5 * (double)nn * nn * es * batch);
   if (ctx->use_trsv_coop) {

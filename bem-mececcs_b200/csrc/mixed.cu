@@ -305,7 +305,7 @@ int sweep(bem_ctx* ctx, const double zge[2], const double zcs[2], const double z
       const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
       cudaGraphExec_t ex = nullptr;
       bool ok = erc == BEM_OK && ce == cudaSuccess && g &&
-                cudaGraphInstantiate(&ex, g, 0) == cudaSuccess &&
+                cudaGraphInstantiate(&ex, g, cudaGraphInstantiateFlagUseNodePriority) == cudaSuccess &&
                 dyn_graph_nodes(ctx, g, ctx->sweep_dyn_nodes) == BEM_OK;
       cudaGetLastError();
       if (ok) {
@@ -442,6 +442,7 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
     bem_ctx* w = nullptr;
     const int rc = bem_ctx_create(d->device, &w);
     if (rc) return fail(d, rc, "bem_batch_solve: worker context");
+    w->lu_lookahead = false;  // the workers' streams overlap each other
     d->workers.push_back(w);
   }
   // Plan: size classes in sorted order, round-robin over the workers, each
