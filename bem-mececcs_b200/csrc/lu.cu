@@ -2111,16 +2111,17 @@ constexpr size_t kLtTile = (size_t)64 * kLtLd * sizeof(float2);
 // kLfragMat floats per 64 x 64 matrix; per problem L11^-1 as a TF32 pair hi +
 // lo, then the earlier panels' L at this panel's rows.
 constexpr int kLfragMat = 64 * 64 * 2, kLfragMats = 2 + kGroupMaps;
-__device__ __forceinline__ int lfrag_index(int i, int t, int part) {
-  return (((((i >> 4) * 8 + (t >> 3)) * 2 + part) * 32 + (i & 7) * 4 + (t & 3)) << 2) + ((i >> 3) & 1) + 2 * ((t >> 2) & 1);
+// A lane's fragment: rows g and g + 8 of columns t4 and t4 + 4.
+__device__ __forceinline__ void tf32_fragment(const float2 (&v)[4], float4& re, float4& im) {
+  re = make_float4(__uint_as_float(to_tf32(v[0].x)), __uint_as_float(to_tf32(v[1].x)), __uint_as_float(to_tf32(v[2].x)),
+                   __uint_as_float(to_tf32(v[3].x)));
+  im = make_float4(__uint_as_float(to_tf32(v[0].y)), __uint_as_float(to_tf32(v[1].y)), __uint_as_float(to_tf32(v[2].y)),
+                   __uint_as_float(to_tf32(v[3].y)));
 }
 
 // For the panel at (k, k) of width w, once per panel and problem
 // (blockIdx.y).  blockIdx.x = 0: L11^-1 (unit lower, zero-padded to 64 x 64),
-// by 16 x 16 diagonal blocks (a warp each, lane = column), then [[X11, 0],
-// [X21, X22]] with X21 = -X22 L21 X11 at 16 and at 32 (one output per thread
-// of 1024); the zero block above the diagonal (rows 0-31, columns 32-63)
-// holds the intermediate L21 X11.
+// by 8 x 8 diagonal blocks, doubled three times.
 // In a group of gsize panels (panel gi of it, gi >= 0) the group's row maps
 // are kept here too: map j (of the group's panel j < gsize - 1) gives, for a
 // position x now, the position the row held after panel j (where L of panel
@@ -2149,24 +2150,18 @@ __global__ void __launch_bounds__(1024) k_l11_inv(const float2* __restrict__ Aba
     }
     if (tid < 64) s_row[tid] = tid < w ? val : -1;
     __syncthreads();  // every read before any write
+    // panel j's L at these rows, a thread per lane's fragment of a (row tile, k step)
+    const float2* Lj = A + (size_t)(k - 64 * (gi - j) + 8 * (warp & 7) + (lane & 3)) * lda;
+    const int i0 = 16 * (warp >> 3) + (lane >> 2), r0 = s_row[i0], r1 = s_row[i0 + 8];
+    const float2 zero = make_float2(0.f, 0.f);
+    const float2 v[4] = {r0 >= 0 ? Lj[r0] : zero, r1 >= 0 ? Lj[r1] : zero, r0 >= 0 ? Lj[4 * lda + r0] : zero,
+                         r1 >= 0 ? Lj[4 * lda + r1] : zero};
+    float4 re, im;
+    tf32_fragment(v, re, im);
+    float4* o = reinterpret_cast<float4*>(out + (size_t)(2 + j) * kLfragMat) + warp * 64 + lane;
+    o[0] = re;
+    o[32] = im;
     if (dst >= 0) gm[dst] = val;
-    const int kj = k - 64 * (gi - j);  // panel j's first column
-    float* s_f = reinterpret_cast<float*>(smem_raw);
-    float2 v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = tid + q * 1024, i = idx & 63, t = idx >> 6, r = s_row[i];
-      v[q] = r >= 0 ? A[(size_t)(kj + t) * lda + r] : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = tid + q * 1024, i = idx & 63, t = idx >> 6;
-      s_f[lfrag_index(i, t, 0)] = __uint_as_float(to_tf32(v[q].x));
-      s_f[lfrag_index(i, t, 1)] = __uint_as_float(to_tf32(v[q].y));
-    }
-    __syncthreads();
-    float4* o = reinterpret_cast<float4*>(out + (size_t)(2 + j) * kLfragMat);
-    for (int idx = tid; idx < kLfragMat / 4; idx += 1024) o[idx] = reinterpret_cast<const float4*>(s_f)[idx];
     return;
   }
   // L11 (unit lower, w x w at (k, k)) into registers first: these loads
@@ -2189,18 +2184,18 @@ __global__ void __launch_bounds__(1024) k_l11_inv(const float2* __restrict__ Aba
     s_inv[i * kLtLd + c] = make_float2(i == c ? 1.f : 0.f, 0.f);
   }
   __syncthreads();
-  // X = L11^-1 by blocks: the four 16 x 16 diagonal blocks (a warp each,
-  // lane = column), then [[X11, 0], [X21, X22]] with X21 = -X22 L21 X11 at
-  // 16 and at 32; the zero block above the diagonal (rows 0-31, columns
-  // 32-63 of s_inv) holds the intermediate L21 X11.
+  // X = L11^-1 by blocks: the eight 8 x 8 diagonal blocks (a warp each, lane =
+  // column), then [[X11, 0], [X21, X22]] with X21 = -X22 L21 X11 at 8, 16 and
+  // 32; the zero block above the diagonal (rows 0-31, columns 32-63 of s_inv)
+  // holds the intermediate L21 X11.
   auto at = [&](float2* M, int i, int j) -> float2& { return M[i * kLtLd + j]; };
-  if (warp < 4 && lane < 16) {
-    const int b0 = 16 * warp, c = lane;
-    zf x[16];
+  if (warp < 8 && lane < 8) {
+    const int b0 = 8 * warp, c = lane;
+    zf x[8];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) x[i] = zf{i == c ? 1.f : 0.f, 0.f};
+    for (int i = 0; i < 8; ++i) x[i] = zf{i == c ? 1.f : 0.f, 0.f};
 #pragma unroll
-    for (int i = 1; i < 16; ++i) {
+    for (int i = 1; i < 8; ++i) {
       zf acc{0.f, 0.f}, acc2{0.f, 0.f};  // two chains: even and odd t
 #pragma unroll
       for (int t = 0; t < i; ++t) {  // x_t = 0 for t < c
@@ -2210,63 +2205,65 @@ __global__ void __launch_bounds__(1024) k_l11_inv(const float2* __restrict__ Aba
       if (i > c) x[i] = zf{acc.re + acc2.re, acc.im + acc2.im};
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) at(s_inv, b0 + i, b0 + c) = make_float2(x[i].re, x[i].im);
+    for (int i = 0; i < 8; ++i) at(s_inv, b0 + i, b0 + c) = make_float2(x[i].re, x[i].im);
   }
   __syncthreads();
-  // X21 = -X22 (L21 X11) for two 16-blocks (h = 16) and then one 32-block (h = 32)
-  for (int h = 16; h <= 32; h *= 2) {
-    const int npair = 64 / (2 * h), outs = npair * h * h;
-    for (int idx = tid; idx < outs; idx += blockDim.x) {  // T = L21 X11 into the scratch block
-      const int pp = idx / (h * h), i = (idx / h) % h, j = idx % h, o = pp * 2 * h;
-      zf acc{0.f, 0.f}, acc2{0.f, 0.f};  // two chains: even and odd t
+  // 2 x 2 outputs per thread (one per thread read four times as much shared
+  // memory) and little code, since a launch runs it once and every line of it
+  // costs an instruction-cache miss (16 x 16 diagonal blocks unrolled were
+  // five times as long).  With the fragments written straight from the rows:
+  // 32 factorisations of 720 unknowns 1.68 -> 1.645 ms, 10 of 2871 8.33 -> 8.21.
+#pragma unroll 1
+  for (int h = 8; h <= 32; h *= 2) {
+    const int hh = h / 2, outs = (64 / (2 * h)) * hh * hh;
+    const int pp = tid / (hh * hh), i = 2 * ((tid / hh) % hh), j = 2 * (tid % hh), o = pp * 2 * h;
+    // out (2 x 2) = sg * sum_t P(., t) Q(t, .), even and odd t apart
+    auto product = [&](const float2* P, const float2* Q, float2* out, float sg) {
+      zf acc[2][4] = {};
+#pragma unroll 2
       for (int t = 0; t < h; t += 2) {
-        const float2 l = at(s_b, o + h + i, o + t), x = at(s_inv, o + t, o + j);
-        const float2 l2 = at(s_b, o + h + i, o + t + 1), x2 = at(s_inv, o + t + 1, o + j);
-        cfms(acc, zf{l.x, l.y}, zf{x.x, x.y});
-        cfms(acc2, zf{l2.x, l2.y}, zf{x2.x, x2.y});
-      }
-      at(s_inv, pp * h + i, 32 + j) = make_float2(-acc.re - acc2.re, -acc.im - acc2.im);  // acc = -T
-    }
-    __syncthreads();
-    for (int idx = tid; idx < outs; idx += blockDim.x) {  // X21 = -X22 T
-      const int pp = idx / (h * h), i = (idx / h) % h, j = idx % h, o = pp * 2 * h;
-      zf acc{0.f, 0.f}, acc2{0.f, 0.f};
-      for (int t = 0; t < h; t += 2) {
-        const float2 x = at(s_inv, o + h + i, o + h + t), tt = at(s_inv, pp * h + t, 32 + j);
-        const float2 x2 = at(s_inv, o + h + i, o + h + t + 1), tt2 = at(s_inv, pp * h + t + 1, 32 + j);
-        cfms(acc, zf{x.x, x.y}, zf{tt.x, tt.y});
-        cfms(acc2, zf{x2.x, x2.y}, zf{tt2.x, tt2.y});
-      }
-      at(s_inv, o + h + i, o + j) = make_float2(acc.re + acc2.re, acc.im + acc2.im);  // acc = -X22 T
-    }
-    __syncthreads();
-  }
-  for (int idx = tid; idx < 32 * 32; idx += blockDim.x) at(s_inv, idx >> 5, 32 + (idx & 31)) = make_float2(0.f, 0.f);
-  __syncthreads();
-  // fragments, through the memory of L11 (hi) and the inverse's own (lo)
-  float* s_hi = reinterpret_cast<float*>(s_b);
-  float2 x[4];
+        const float4 p[2] = {*reinterpret_cast<const float4*>(P + t), *reinterpret_cast<const float4*>(P + kLtLd + t)};
+        const float4 q0 = *reinterpret_cast<const float4*>(Q + t * kLtLd);
+        const float4 q1 = *reinterpret_cast<const float4*>(Q + (t + 1) * kLtLd);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int idx = tid + q * 1024;
-    x[q] = s_inv[(idx >> 6) * kLtLd + (idx & 63)];
-  }
-  __syncthreads();
-  float* s_lo = reinterpret_cast<float*>(s_inv);
+        for (int r = 0; r < 2; ++r) {
+          cfms(acc[0][2 * r], zf{p[r].x, p[r].y}, zf{q0.x, q0.y});
+          cfms(acc[0][2 * r + 1], zf{p[r].x, p[r].y}, zf{q0.z, q0.w});
+          cfms(acc[1][2 * r], zf{p[r].z, p[r].w}, zf{q1.x, q1.y});
+          cfms(acc[1][2 * r + 1], zf{p[r].z, p[r].w}, zf{q1.z, q1.w});
+        }
+      }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int idx = tid + q * 1024, i = idx >> 6, t = idx & 63;
-    const float re = __uint_as_float(to_tf32(x[q].x)), im = __uint_as_float(to_tf32(x[q].y));
-    s_hi[lfrag_index(i, t, 0)] = re;
-    s_hi[lfrag_index(i, t, 1)] = im;
-    s_lo[lfrag_index(i, t, 0)] = __uint_as_float(to_tf32(x[q].x - re));
-    s_lo[lfrag_index(i, t, 1)] = __uint_as_float(to_tf32(x[q].y - im));
+      for (int r = 0; r < 2; ++r) {
+        const zf *e = &acc[0][2 * r], *d = &acc[1][2 * r];
+        *reinterpret_cast<float4*>(out + r * kLtLd) = make_float4(-sg * (e[0].re + d[0].re), -sg * (e[0].im + d[0].im),
+                                                                  -sg * (e[1].re + d[1].re), -sg * (e[1].im + d[1].im));
+      }
+    };
+    float2* const scratch = &at(s_inv, pp * h, 32);
+    if (tid < outs) product(&at(s_b, o + h + i, o), &at(s_inv, o, o + j), scratch + i * kLtLd + j, 1.f);
+    __syncthreads();
+    if (tid < outs) product(&at(s_inv, o + h + i, o + h), scratch + j, &at(s_inv, o + h + i, o + j), -1.f);
+    __syncthreads();
   }
-  __syncthreads();
-  float4* o = reinterpret_cast<float4*>(out);
-  for (int idx = tid; idx < kLfragMat / 4; idx += 1024) {
-    o[idx] = reinterpret_cast<const float4*>(s_hi)[idx];
-    o[kLfragMat / 4 + idx] = reinterpret_cast<const float4*>(s_lo)[idx];
+  // fragments of the lower triangle, hi and lo, a thread per lane's of a (row tile, k step)
+  {
+    const int i0 = 16 * (warp >> 3) + (lane >> 2), t0 = 8 * (warp & 7) + (lane & 3);
+    float2 v[4], lo[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + 8 * (e & 1), t = t0 + 4 * (e >> 1);
+      v[e] = t <= i ? s_inv[i * kLtLd + t] : make_float2(0.f, 0.f);
+      lo[e] = make_float2(v[e].x - __uint_as_float(to_tf32(v[e].x)), v[e].y - __uint_as_float(to_tf32(v[e].y)));
+    }
+    float4 re, im;
+    float4* o = reinterpret_cast<float4*>(out) + warp * 64 + lane;
+    tf32_fragment(v, re, im);
+    o[0] = re;
+    o[32] = im;
+    tf32_fragment(lo, re, im);
+    o[kLfragMat / 4] = re;
+    o[kLfragMat / 4 + 32] = im;
   }
 }
 
