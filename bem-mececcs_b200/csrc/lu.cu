@@ -4126,17 +4126,22 @@ static int trsv_cl(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, in
   const int stages = (int)std::min<size_t>(6, (kSmem - fixed) / stage);
   CUtensorMap tm;
   if (!make_rows_map(&tm, A, nn, lda, bstride, batch, 64)) return BEM_OK;
-  auto need = [&](auto*& p, size_t& cap, size_t bytes) -> int {
-    if (cap >= bytes) return BEM_OK;
+  // (no memory for this form's tables: the cooperative kernels, which need less)
+  auto need = [&](auto*& p, size_t& cap, size_t bytes) {
+    if (cap >= bytes) return true;
     dev_free(ctx, p);
     p = nullptr;
     cap = 0;
-    BEM_CUDA(ctx, dev_alloc(ctx, &p, bytes));
+    if (dev_alloc(ctx, &p, bytes) != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();
+      return false;
+    }
     cap = bytes;
-    return BEM_OK;
+    return true;
   };
-  int rc = need(L.tinv, L.tinv_bytes, (size_t)batch * (npan + nb) * stage);
-  if (rc) return rc;
+  if (L.tinv_bytes < (size_t)batch * (npan + nb) * stage) L.tinv_valid = L.uinv_valid = false;
+  if (!need(L.tinv, L.tinv_bytes, (size_t)batch * (npan + nb) * stage)) return BEM_OK;
   float2* A2 = static_cast<float2*>(A);
   constexpr size_t kInvSmem = 2 * kLtTile;
   BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_tri_inv_cl), kInvSmem));
@@ -4147,19 +4152,18 @@ static int trsv_cl(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, in
     return BEM_OK;
   };
   if (!L.uinv_valid) {
-    rc = invert(npan, nb);
+    const int rc = invert(npan, nb);
     if (rc) return rc;
     L.uinv_valid = true;
     L.tinv_valid = false;
   }
   if (forward && !L.lperm_valid) {
-    rc = need(L.rmap, L.rmap_bytes, ((size_t)(npan + 1) * nn + npan) * batch * sizeof(int));
-    if (rc) return rc;
+    if (!need(L.rmap, L.rmap_bytes, ((size_t)(npan + 1) * nn + npan) * batch * sizeof(int))) return BEM_OK;
     int* moved = L.rmap + (size_t)(npan + 1) * nn * batch;
     const size_t msm = (size_t)2 * nn * sizeof(int), psm = (size_t)nn * sizeof(float2);
     BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_row_maps), msm));
     BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_lperm), psm));
-    rc = invert(0, npan);
+    const int rc = invert(0, npan);
     if (rc) return rc;
     k_row_maps<<<batch, 1024, msm, ctx->stream>>>(nn, npan, batch, L.perm, L.rmap, moved);
     if (npan > 1)
