@@ -424,6 +424,24 @@ int ensure_batchbuf(bem_ctx* d, const BatchNeed& q, bool mixed) {
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// Worker i of a batch call takes the larger classes the smaller i is, and its
+// stream the higher priority: the largest classes' chains of panels decide when
+// the call ends, the rest fills the SMs they leave.  Smallest class first and
+// equal priorities: 96 meshes of n = 72..1800 17.6 ms against 17.2, 40 of
+// 180..900 3.98 / 3.48, 12 of 90..1500 5.08 / 4.45, plain form, 48 of 90..1200
+// 7.79 / 6.90.
+int worker_priority(bem_ctx* w, int i) {
+  int lo = 0, hi = 0;
+  cudaStream_t s = nullptr;
+  BEM_CUDA(w, cudaDeviceGetStreamPriorityRange(&lo, &hi));
+  BEM_CUDA(w, cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, std::min(lo, hi + i)));
+  const cudaError_t e = cudaStreamSynchronize(w->own_stream);  // its allocations
+  cudaStreamDestroy(w->own_stream);
+  w->own_stream = w->stream = s;
+  BEM_CUDA(w, e);
+  return BEM_OK;
+}
+
 }  // namespace
 
 constexpr int kBatchWorkers = 8;
@@ -437,20 +455,25 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
   std::vector<int> order(nprob);
   for (int i = 0; i < nprob; ++i) order[i] = i;
   std::sort(order.begin(), order.end(), [&](int a, int b) { return probs[a]->mesh.nbe < probs[b]->mesh.nbe; });
-  // Worker contexts: classes go round-robin to their streams and run concurrently.
+  // Worker contexts: classes go round-robin to their streams, the largest to
+  // the first, and run concurrently.
   while ((int)d->workers.size() < kBatchWorkers) {
     bem_ctx* w = nullptr;
-    const int rc = bem_ctx_create(d->device, &w);
+    int rc = bem_ctx_create(d->device, &w);
+    if (!rc) {
+      rc = worker_priority(w, (int)d->workers.size());
+      if (rc) bem_ctx_destroy(w);
+    }
     if (rc) return fail(d, rc, "bem_batch_solve: worker context");
     w->lu_lookahead = false;  // the workers' streams overlap each other
     d->workers.push_back(w);
   }
-  // Plan: size classes in sorted order, round-robin over the workers, each
-  // worker's buffers sized once for all its classes (no allocation between
-  // launches).
+  // Plan: size classes in sorted order; each worker's buffers are sized once
+  // for all its classes (no allocation between launches).
   struct Cls {
     int g0, g1, npad;
     size_t sol;  // offset of its solutions in the pinned staging, in double2
+    size_t diag, rhs;
   };
   std::vector<Cls> plan;
   std::vector<BatchNeed> need_w(kBatchWorkers);
@@ -470,11 +493,13 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
       diag += (size_t)9 * probs[order[k]]->mesh.nbe;
       rhs += (size_t)rhs_chunks(probs[order[k]]) * 3 * probs[order[k]]->mesh.nbe;
     }
-    need_w[plan.size() % kBatchWorkers].add(npad, g1 - g0, diag, rhs);
-    plan.push_back({g0, g1, npad, sol_total});
+    plan.push_back({g0, g1, npad, sol_total, diag, rhs});
     sol_total += (size_t)(g1 - g0) * npad;
     g0 = g1;
   }
+  auto worker_of = [&](int ncls) { return ((int)plan.size() - 1 - ncls) % kBatchWorkers; };
+  for (int i = 0; i < (int)plan.size(); ++i)
+    need_w[worker_of(i)].add(plan[i].npad, plan[i].g1 - plan[i].g0, plan[i].diag, plan[i].rhs);
   for (int w = 0; w < kBatchWorkers; ++w) {
     if (need_w[w].a_elems == 0) continue;
     const int rc = ensure_batchbuf(d->workers[w], need_w[w], mixed);
@@ -508,8 +533,9 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
   std::vector<int> class_of(nprob), slot_of(nprob);
   for (bem_ctx* w : d->workers) BEM_CUDA(w, cudaMemsetAsync(w->d_status, 0, ST_COUNT * sizeof(int), w->stream));
   std::vector<GroupMember> mem;
-  for (int ncls = 0; ncls < (int)plan.size(); ++ncls) {
-    bem_ctx* wk = d->workers[ncls % kBatchWorkers];
+  // the largest class first: its chain of panels is the longest
+  for (int ncls = (int)plan.size() - 1; ncls >= 0; --ncls) {
+    bem_ctx* wk = d->workers[worker_of(ncls)];
     const int g0 = plan[ncls].g0, g1 = plan[ncls].g1, npad = plan[ncls].npad;
     const int B = g1 - g0;
     int rc = BEM_OK;
