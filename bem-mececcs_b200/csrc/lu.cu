@@ -3741,7 +3741,8 @@ static int panel_cs_min(int m, int cs_max) {
 static int panel_resident(bem_ctx* ctx, int cs);
 
 // The panel of m rows of `batch` problems: more CTAs per problem than the
-// fewest while all problems' clusters stay resident together and the rows per
+// fewest while all problems' clusters (and those of other workers of a batch
+// call, panel_share) stay resident together and the rows per
 // CTA are above about 230 (FP32) or 100 (FP64), below which a step no longer
 // gets faster (720 rows: 82 us on 8 CTAs, 86 on 4, 98 on 2).
 template <typename R>
@@ -3752,7 +3753,7 @@ static PanelShape panel_shape(bem_ctx* ctx, int m, int batch) {
   s.sl = panel_slice<R>(panel_even((m + cs - 1) / cs));
   if (s.sl == 0 || panel_even((m + cs - 1) / cs) > kPanelIpRows<R>) return s;
   const int enough = sizeof(R) == 4 ? 230 : 100;
-  while (cs < cs_max && m > enough * cs && batch <= panel_resident(ctx, 2 * cs)) cs *= 2;
+  while (cs < cs_max && m > enough * cs && batch * ctx->panel_share <= panel_resident(ctx, 2 * cs)) cs *= 2;
   if (!ctx->small_clusters) cs = cs_max;
   s.cs = cs;
   s.rp = panel_even((m + cs - 1) / cs);

@@ -533,9 +533,16 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
   std::vector<int> class_of(nprob), slot_of(nprob);
   for (bem_ctx* w : d->workers) BEM_CUDA(w, cudaMemsetAsync(w->d_status, 0, ST_COUNT * sizeof(int), w->stream));
   std::vector<GroupMember> mem;
+  // A panel of few CTAs takes a little longer (720 rows: 98 us on 2, 82 on 8) and
+  // holds far fewer SMs: with many problems at once the SMs are what is short.
+  // Panels sized as if alone, or as 2, 4 and 8 at a time: 96 problems 17.25,
+  // 16.67, 16.30, 16.20 ms; 48 (plain) 6.95, 6.67, 6.67, 6.66; 40 3.50, 3.49,
+  // 3.55, 3.53; 12 4.45, 4.48, 4.48, 4.47.
+  const int share = std::max(1, std::min(kBatchWorkers, nprob / 24));
   // the largest class first: its chain of panels is the longest
   for (int ncls = (int)plan.size() - 1; ncls >= 0; --ncls) {
     bem_ctx* wk = d->workers[worker_of(ncls)];
+    wk->panel_share = share;
     const int g0 = plan[ncls].g0, g1 = plan[ncls].g1, npad = plan[ncls].npad;
     const int B = g1 - g0;
     int rc = BEM_OK;
