@@ -494,6 +494,7 @@ class Server {
         fresh = &slots_.back();
       }
       int st = bem_ctx_create(device_, &fresh->ctx);
+      if (st == BEM_OK) fresh->ctx->lu_lookahead = false;  // the slots' streams overlap each other
       if (st == BEM_OK)
         st = bem_mesh_upload(fresh->ctx, m.n, m.nbe, m.np, m.npg, m.cone.data(), m.cx.data(), m.cy.data(),
                              m.cz.data(), m.cxm.data(), m.cym.data(), m.czm.data(), m.etas.data(), m.gi.data(),
