@@ -141,13 +141,14 @@ class Context:
         except Exception:
             pass
 
-    INT_OPTIONS = ("gemm_ctas", "trsv_ctas", "wait_limit_ms")
+    INT_OPTIONS = ("gemm_ctas", "trsv_ctas", "wait_limit_ms", "fail_alloc")
 
     def set_option(self, name: str, value) -> None:
         """bem_ctx_set_option: switches tcgen05, trsv_coop, lu_pairs, lu_quads,
         f64_pairs, tc_pair, panel_calu, panel_push, panel_async, laswp_tc, trsv_inv, graphs; CTA
         budgets gemm_ctas, trsv_ctas (0 = device); wait_limit_ms, the bound of
-        every device-side wait (1..60000, default 2000)."""
+        every device-side wait (1..60000, default 2000); fail_alloc, the device
+        allocation that fails (self-test)."""
         v = int(value) if name in self.INT_OPTIONS else int(bool(value))
         self.check(self.L.bem_ctx_set_option(self.h, name.encode(), v), "bem_ctx_set_option")
 

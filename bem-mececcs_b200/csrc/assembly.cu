@@ -644,6 +644,7 @@ int launch_static(bem_ctx* ctx, const double c[4], int compute_gest, double* hes
   if (chunks > ctx->static_chunks) {
     if (ctx->static_part) dev_free(ctx, ctx->static_part);
     ctx->static_part = nullptr;
+    ctx->static_chunks = 0;
     BEM_CUDA(ctx, dev_alloc(ctx, &ctx->static_part, (size_t)chunks * m.nbe * 9 * sizeof(double)));
     ctx->static_chunks = chunks;
   }
@@ -893,6 +894,7 @@ int launch_dynamic(bem_ctx* ctx, const double zge[2], const double zcs[2], const
   if (chunks > s.rhs_chunks) {
     if (s.rhs_part) dev_free(ctx, s.rhs_part);
     s.rhs_part = nullptr;
+    s.rhs_chunks = 0;
     BEM_CUDA(ctx, dev_alloc(ctx, &s.rhs_part, (size_t)chunks * s.nn * sizeof(double2)));
     s.rhs_chunks = chunks;
   }

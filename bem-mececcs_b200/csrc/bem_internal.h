@@ -244,6 +244,8 @@ struct bem_ctx {
   int wait_limit_ms = 2000;   // bound of every device-side wait (copy of the device word)
   std::unordered_map<long long, int> lockstep_cache;  // lu_lockstep_capacity by (size, precision)
   unsigned long long alloc_epoch = 0;  // device allocations so far (dev_alloc)
+  int fail_alloc = 0;                  // option fail_alloc: the allocation, counted from now, that fails
+  int* fail_ctr = &fail_alloc;         // (bem_batch_solve's workers: the driver's)
   unsigned long long sg_epoch = 0;     // alloc_epoch when the sweep step was captured
 };
 
@@ -262,10 +264,12 @@ int cuda_fail(bem_ctx* ctx, cudaError_t e, const char* what);
 // (bem_ctx_set_stream) waits for its old one first.  Every allocation also
 // advances ctx->alloc_epoch: a captured sweep step names the buffers it was
 // captured with and is replayed only while no buffer of the context has been
-// (re)allocated since.
+// (re)allocated since.  A call that fails here must leave every buffer it was
+// replacing empty and its capacity zero: a later, smaller call trusts them.
 template <typename T>
 cudaError_t dev_alloc(bem_ctx* ctx, T** p, size_t bytes) {
   ++ctx->alloc_epoch;
+  if (*ctx->fail_ctr > 0 && --*ctx->fail_ctr == 0) return cudaErrorMemoryAllocation;
   return cudaMallocAsync(reinterpret_cast<void**>(p), bytes, ctx->stream);
 }
 void dev_free(bem_ctx* ctx, void* p);

@@ -77,15 +77,19 @@ static int ensure_system(bem_ctx* ctx, int nn, bool preswap) {
   System& s = ctx->sys;
   if (s.nn != nn || !s.A) {
     free_system(ctx, s);
+    const int nbe = (nn + 2) / 3;
+    cudaError_t e = dev_alloc(ctx, &s.A, (size_t)nn * (size_t)(nn + 1) * sizeof(double2));
+    if (e == cudaSuccess) e = dev_alloc(ctx, &s.diag_h, (size_t)nbe * 9 * sizeof(double2));
+    if (e == cudaSuccess) e = dev_alloc(ctx, &s.diag_g, (size_t)nbe * 9 * sizeof(double2));
+    if (e != cudaSuccess) {
+      free_system(ctx, s);
+      return cuda_fail(ctx, e, "buffers of the system");
+    }
     s.nn = nn;
     s.lda = (size_t)nn;
-    BEM_CUDA(ctx, dev_alloc(ctx, &s.A, s.lda * (size_t)(nn + 1) * sizeof(double2)));
-    const int nbe = (nn + 2) / 3;
-    BEM_CUDA(ctx, dev_alloc(ctx, &s.diag_h, (size_t)nbe * 9 * sizeof(double2)));
-    BEM_CUDA(ctx, dev_alloc(ctx, &s.diag_g, (size_t)nbe * 9 * sizeof(double2)));
   }
-  if (preswap && !s.zh_pre) {
-    BEM_CUDA(ctx, dev_alloc(ctx, &s.zh_pre, (size_t)nn * nn * sizeof(double2)));
+  if (preswap && !(s.zh_pre && s.zg_pre)) {
+    if (!s.zh_pre) BEM_CUDA(ctx, dev_alloc(ctx, &s.zh_pre, (size_t)nn * nn * sizeof(double2)));
     BEM_CUDA(ctx, dev_alloc(ctx, &s.zg_pre, (size_t)nn * nn * sizeof(double2)));
   }
   return BEM_OK;
@@ -276,6 +280,7 @@ int bem_mesh_upload(bem_ctx* ctx, int n, int nbe, int np, int npg, const int* co
   cudaSetDevice(ctx->device);
   BEM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   free_mesh(ctx, ctx->mesh);
+  ctx->have_mesh = ctx->have_hest = ctx->have_gest = ctx->have_dyn = false;  // until the new one is complete
   Mesh& m = ctx->mesh;
   m.n = n;
   m.nbe = nbe;
@@ -295,8 +300,12 @@ int bem_mesh_upload(bem_ctx* ctx, int n, int nbe, int np, int npg, const int* co
   const size_t nd = (size_t)3 * np + 6 * (size_t)n;
   double* d_raw = nullptr;
   int* d_cone = nullptr;
-  BEM_CUDA(ctx, dev_alloc(ctx, &d_raw, nd * sizeof(double)));
-  BEM_CUDA(ctx, dev_alloc(ctx, &d_cone, (size_t)4 * n * sizeof(int)));
+  cudaError_t ae = dev_alloc(ctx, &d_raw, nd * sizeof(double));
+  if (ae == cudaSuccess) ae = dev_alloc(ctx, &d_cone, (size_t)4 * n * sizeof(int));
+  if (ae != cudaSuccess) {
+    dev_free(ctx, d_raw);
+    return cuda_fail(ctx, ae, "staging of the mesh");
+  }
   double *dcx = d_raw, *dcy = dcx + np, *dcz = dcy + np, *detas = dcz + np, *dcxm = detas + 3 * (size_t)n,
          *dcym = dcxm + n, *dczm = dcym + n;
   cudaStream_t st = ctx->stream;
@@ -315,8 +324,6 @@ int bem_mesh_upload(bem_ctx* ctx, int n, int nbe, int np, int npg, const int* co
   if (rc) return rc;
   int flags[2];
   BEM_CUDA(ctx, cudaMemcpy(flags, ctx->d_status + ST_COUNT, sizeof flags, cudaMemcpyDeviceToHost));
-  ctx->have_mesh = true;
-  ctx->have_hest = ctx->have_gest = ctx->have_dyn = false;
   // Per-mesh buffers sized by nbe are reallocated on the next use.
   dev_free(ctx, ctx->zdfi);
   dev_free(ctx, ctx->kode);
@@ -335,6 +342,7 @@ int bem_mesh_upload(bem_ctx* ctx, int n, int nbe, int np, int npg, const int* co
   // Remember the degenerate flags: [0] any element, [1] boundary elements.
   ctx->mesh_flag_all = flags[0];
   ctx->mesh_flag_bnd = flags[1];
+  ctx->have_mesh = true;
   return BEM_OK;
 }
 
@@ -402,10 +410,8 @@ int bem_dyn_upload(bem_ctx* ctx, const double* zdfi, const int* kode) {
   if (!ctx->have_mesh) return fail(ctx, BEM_ERR_STATE, "bem_dyn_upload before bem_mesh_upload");
   cudaSetDevice(ctx->device);
   const int nn = 3 * ctx->mesh.nbe;
-  if (!ctx->zdfi) {
-    BEM_CUDA(ctx, dev_alloc(ctx, &ctx->zdfi, (size_t)nn * sizeof(double2)));
-    BEM_CUDA(ctx, dev_alloc(ctx, &ctx->kode, (size_t)nn * sizeof(int)));
-  }
+  if (!ctx->zdfi) BEM_CUDA(ctx, dev_alloc(ctx, &ctx->zdfi, (size_t)nn * sizeof(double2)));
+  if (!ctx->kode) BEM_CUDA(ctx, dev_alloc(ctx, &ctx->kode, (size_t)nn * sizeof(int)));
   BEM_CUDA(ctx, cudaMemcpyAsync(ctx->zdfi, zdfi, (size_t)nn * sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
   BEM_CUDA(ctx, cudaMemcpyAsync(ctx->kode, kode, (size_t)nn * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   ctx->h_zdfi.assign(zdfi, zdfi + 2 * (size_t)nn);
@@ -516,9 +522,14 @@ int bem_static_solve(bem_ctx* ctx, const double c[4], double ge, const int* kode
   double* Gs = nullptr;
   double* d_dfi = nullptr;
   int* d_kode = nullptr;
-  BEM_CUDA(ctx, dev_alloc(ctx, &Gs, (size_t)nn * nn * sizeof(double)));
-  BEM_CUDA(ctx, dev_alloc(ctx, &d_dfi, (size_t)nn * sizeof(double)));
-  BEM_CUDA(ctx, dev_alloc(ctx, &d_kode, (size_t)nn * sizeof(int)));
+  cudaError_t ae = dev_alloc(ctx, &Gs, (size_t)nn * nn * sizeof(double));
+  if (ae == cudaSuccess) ae = dev_alloc(ctx, &d_dfi, (size_t)nn * sizeof(double));
+  if (ae == cudaSuccess) ae = dev_alloc(ctx, &d_kode, (size_t)nn * sizeof(int));
+  if (ae != cudaSuccess) {
+    dev_free(ctx, Gs);
+    dev_free(ctx, d_dfi);
+    return cuda_fail(ctx, ae, "buffers of the static solve");
+  }
   BEM_CUDA(ctx, cudaMemcpyAsync(d_dfi, dfi, (size_t)nn * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   BEM_CUDA(ctx, cudaMemcpyAsync(d_kode, kode, (size_t)nn * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   BEM_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, ST_COUNT * sizeof(int), ctx->stream));
@@ -626,10 +637,12 @@ static bool* option_slot(bem_ctx* ctx, const char* name) {
 }
 
 // Integer options: CTA budgets for a context that shares its GPU with
-// another one running at the same time (0 = the whole device).
+// another one running at the same time (0 = the whole device), and the
+// allocation failure of the tests.
 static int* int_option_slot(bem_ctx* ctx, const char* name) {
   if (!strcmp(name, "gemm_ctas")) return &ctx->gemm_ctas;
   if (!strcmp(name, "trsv_ctas")) return &ctx->trsv_ctas;
+  if (!strcmp(name, "fail_alloc")) return &ctx->fail_alloc;
   return nullptr;
 }
 

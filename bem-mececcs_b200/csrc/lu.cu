@@ -3501,26 +3501,26 @@ int lu_ensure_workspace(bem_ctx* ctx, int nn, int batch) {
   if (L.cap_nn >= nn && L.cap_batch >= batch && L.ipiv) return BEM_OK;
   dev_free(ctx, L.ipiv);
   dev_free(ctx, L.perm);
+  dev_free(ctx, L.pstart);
+  dev_free(ctx, L.panel_u);
   L.ipiv = nullptr;
   L.perm = nullptr;
+  L.pstart = nullptr;
+  L.panel_u = nullptr;
+  L.cap_nn = L.cap_batch = 0;
+  L.panels.clear();  // the last factorisation's lists are gone
   BEM_CUDA(ctx, dev_alloc(ctx, &L.ipiv, (size_t)nn * batch * sizeof(int)));
   const int max_panels = (nn + 15) / 16 + 1;
   BEM_CUDA(ctx, dev_alloc(ctx, &L.perm, (size_t)max_panels * kPermStride * batch * sizeof(int)));
-  dev_free(ctx, L.pstart);
-  L.pstart = nullptr;
   BEM_CUDA(ctx, dev_alloc(ctx, &L.pstart, (size_t)(max_panels + 1) * sizeof(int)));
-  dev_free(ctx, L.panel_u);
-  L.panel_u = nullptr;
   BEM_CUDA(ctx, dev_alloc(ctx, &L.panel_u, (size_t)batch * 64 * 64 * sizeof(double2)));
+  if (!L.slot_val) BEM_CUDA(ctx, dev_alloc(ctx, &L.slot_val, 2 * kMaxGrid * sizeof(double)));
+  if (!L.slot_row) BEM_CUDA(ctx, dev_alloc(ctx, &L.slot_row, 2 * kMaxGrid * sizeof(int)));
+  if (!L.cand) BEM_CUDA(ctx, dev_alloc(ctx, &L.cand, (size_t)2 * kMaxGrid * 64 * sizeof(double2)));
+  if (!L.drow) BEM_CUDA(ctx, dev_alloc(ctx, &L.drow, 2 * 64 * sizeof(double2)));
+  if (!L.barrier) BEM_CUDA(ctx, dev_alloc(ctx, &L.barrier, sizeof(unsigned)));
   L.cap_nn = nn;
   L.cap_batch = batch;
-  if (!L.slot_val) {
-    BEM_CUDA(ctx, dev_alloc(ctx, &L.slot_val, 2 * kMaxGrid * sizeof(double)));
-    BEM_CUDA(ctx, dev_alloc(ctx, &L.slot_row, 2 * kMaxGrid * sizeof(int)));
-    BEM_CUDA(ctx, dev_alloc(ctx, &L.cand, (size_t)2 * kMaxGrid * 64 * sizeof(double2)));
-    BEM_CUDA(ctx, dev_alloc(ctx, &L.drow, 2 * 64 * sizeof(double2)));
-    BEM_CUDA(ctx, dev_alloc(ctx, &L.barrier, sizeof(unsigned)));
-  }
   return BEM_OK;
 }
 
@@ -3899,6 +3899,8 @@ static int ensure_cublas(bem_ctx* ctx) {
     cublasHandle_t h = nullptr;
     if (cublasCreate(&h) != CUBLAS_STATUS_SUCCESS) return fail(ctx, BEM_ERR_CUDA, "cublasCreate failed");
     ctx->cublas = h;
+  }
+  if (!ctx->cublas_ws) {
     BEM_CUDA(ctx, dev_alloc(ctx, reinterpret_cast<unsigned char**>(&ctx->cublas_ws), kCublasWorkspace));
     BEM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
@@ -4755,7 +4757,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
       look = ctx->crit && (sizeof(R) == 4 ? L.linv_bytes >= 8 * linv_slot * sizeof(float) &&
                                                 L.gmap_bytes >= (size_t)batch * kGroupMaps * nn * sizeof(int) &&
                                                 ctx->tc.lhat2
-                                          : ctx->cublas && ctx->crit_ws && L.lg_cap >= lookahead_lg(nn, batch));
+                                          : ctx->cublas_ws && ctx->crit_ws && L.lg_cap >= lookahead_lg(nn, batch));
     else
       look = sizeof(R) == 4
                  ? (ctx->tc.lhat2 || lookahead_room(ctx, ctx->tc.lrows_cap * kTcKPitch * sizeof(float))) &&

@@ -466,6 +466,7 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
     }
     if (rc) return fail(d, rc, "bem_batch_solve: worker context");
     w->lu_lookahead = false;  // the workers' streams overlap each other
+    w->fail_ctr = d->fail_ctr;
     d->workers.push_back(w);
   }
   // Plan: size classes in sorted order; each worker's buffers are sized once

@@ -157,7 +157,10 @@ int bem_ctx_set_stream(bem_ctx *ctx, void *stream);
  * "wait_limit_ms" (1..60000, default 2000): how long any device-side wait of
  * ctx's kernels (a bulk-copy mbarrier, a cluster mailbox, a software grid
  * barrier) may last before the kernel gives up, records a timeout and
- * returns; the call then reports BEM_ERR_TIMEOUT. */
+ * returns; the call then reports BEM_ERR_TIMEOUT.
+ * "fail_alloc" (failure self-test; 0, the default, none): the n-th device
+ * allocation of the context from now on fails as if memory were exhausted,
+ * once; the option counts down to 0. */
 int bem_ctx_set_option(bem_ctx *ctx, const char *name, int value);
 int bem_ctx_get_option(bem_ctx *ctx, const char *name, int *value);
 const char *bem_status_string(int status);
