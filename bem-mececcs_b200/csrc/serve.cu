@@ -347,12 +347,13 @@ class Server {
     return p;
   }
 
-  // Frees idle slots, least recently used first, until `need` more bytes fit.
-  bool make_room(size_t need) {
+  // Frees idle slots, least recently used first, until `need` more bytes fit;
+  // never `keep`, the slot they are for.
+  bool make_room(size_t need, const Slot* keep = nullptr) {
     while (used_bytes_ + need > budget_) {
       Slot* victim = nullptr;
       for (Slot& s : slots_)
-        if (s.ctx && !s.busy && (!victim || s.last_use < victim->last_use)) victim = &s;
+        if (s.ctx && !s.busy && &s != keep && (!victim || s.last_use < victim->last_use)) victim = &s;
       if (!victim) return false;
       destroy_slot(*victim);
       ++n_evict_;
@@ -464,7 +465,7 @@ class Server {
     }
     if (slot && !rhs_only && (int)batch.size() > slot->cap_probs) {
       // a batch wider than the slot was admitted for: room for the difference, or one problem
-      if (!make_room(per * (batch.size() - slot->cap_probs))) batch.resize(slot->cap_probs);
+      if (!make_room(per * (batch.size() - slot->cap_probs), slot)) batch.resize(slot->cap_probs);
       else {
         used_bytes_ += per * (batch.size() - slot->cap_probs);
         peak_bytes_ = std::max(peak_bytes_, used_bytes_);

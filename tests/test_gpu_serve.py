@@ -147,3 +147,30 @@ def test_same_mesh_sweep_batched_in_lockstep(form):
     assert st["completed"] == len(freqs) and st["max_busy"] >= 2  # several problems in flight together
     for (d0, t0), (d1, t1) in zip(alone, got):
         assert rel(d1, d0) < TOL and rel(t1, t0) < TOL
+
+
+def test_a_wider_batch_keeps_its_own_slot():
+    """An idle slot taken over by a wider batch is the least recently used one
+    when its growth needs room: another slot goes, or the batch stays narrow."""
+    mA, mB = _mesh(14, 12, 6), _mesh(14, 12, 7)
+    bc, kode = _bc(mA, 0.0, 0.0, 1.5)
+    freqs = [0.6, 1.4, 2.3, 3.1]
+    srv = serve.Server(form="mixed", refine=3)
+    a = srv.add_mesh(mA)
+    want, one = [], 0
+    for f in freqs:
+        d, t, info = srv.wait(srv.submit(a, MAT, f, bc, kode))
+        want.append((d, t))
+        one = info["bytes"]
+    srv.close()
+    srv = serve.Server(form="mixed", refine=3, budget_bytes=2.5 * one)
+    a, b = srv.add_mesh(mA), srv.add_mesh(mB)
+    srv.wait(srv.submit(a, MAT, 0.9, bc, kode))
+    srv.wait(srv.submit(b, MAT, 0.9, *_bc(mB, 0.0, 0.0, 1.5)))
+    ids = [srv.submit(a, MAT, f, bc, kode) for f in freqs]
+    got = [srv.wait(i)[:2] for i in ids]
+    st = srv.stats()
+    srv.close()
+    assert st["completed"] == 2 + len(freqs) and st["peak_bytes"] <= 2.5 * one
+    for (d0, t0), (d1, t1) in zip(want, got):
+        assert rel(d1, d0) < TOL and rel(t1, t0) < TOL
