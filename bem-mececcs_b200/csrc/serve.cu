@@ -37,13 +37,20 @@ using Clock = std::chrono::steady_clock;
 
 // Work in flight at once: at most 8 slots (independent solves or lockstep
 // batches) and 16 problems.  Every LU keeps one panel cluster per problem and
-// the device holds about 9 16-CTA clusters at a time; admitting more than
-// that only queues kernels behind each other (measured: 94 concurrent
-// 6480-unknown solves ran 4x slower in total than 16), so a request that fits
-// the memory budget still waits here until a solve finishes.  16 problems let
-// two lockstep batches of a sweep run side by side, one's panels overlapping
-// the other's updates.
+// the device holds 18 8-CTA or about 9 16-CTA clusters at a time; admitting
+// more than that only queues kernels behind each other (measured: 94
+// concurrent 6480-unknown solves ran 4x slower in total than 16), so a request
+// that fits the memory budget still waits here until a solve finishes.
 constexpr int kMaxInflight = 16;
+// Systems above kWideMax unknowns take at most half of the limit in one
+// lockstep batch, although the panel kernel would hold more: two batches of a
+// sweep run side by side, one's panels overlapping the other's updates, and a
+// queued sweep starts beside other work once 8 problems fit instead of waiting
+// for all 16.  128 requests of 6480 unknowns: 182 to 195 solves/s in batches of
+// 8, 144 to 180 in batches of 16; a sweep of 24 submitted beside a
+// 25920-unknown solve has its first result after 35 to 54 ms instead of 32 to
+// 99.  Smaller systems (panels of fewer CTAs) fill the limit.
+constexpr int kWideMax = 2048;
 constexpr int kMaxSlotsBusy = 8;
 constexpr int kDefer = -2;  // try_start: wait for a fuller lockstep batch
 // A request waits for a fuller batch at most this long after its submission,
@@ -417,15 +424,16 @@ class Server {
   }
 
   // Problems in lockstep on one slot for an nn-unknown mesh: the panel
-  // kernel's resident limit, at most kMaxBatch (a context of the server's
-  // own answers the occupancy query and caches it per size).
+  // kernel's resident limit, at most kMaxBatch and, above kWideMax unknowns,
+  // half of the in-flight limit (a context of the server's own answers the
+  // occupancy query and caches it per size).
   int lockstep_cap(int nn) {
     if (!probe_ && bem_ctx_create(device_, &probe_) != BEM_OK) {
       probe_ = nullptr;
       return 1;
     }
     std::lock_guard<std::mutex> g(probe_->mu);
-    return std::max(1, std::min(kMaxBatch, lu_lockstep_capacity(probe_, nn, mixed_)));
+    return std::max(1, std::min(nn > kWideMax ? kMaxInflight / 2 : kMaxBatch, lu_lockstep_capacity(probe_, nn, mixed_)));
   }
 
   // Problems started (the request, and those batched with it), 0 not yet

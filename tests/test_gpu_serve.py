@@ -8,6 +8,8 @@
 * admission respects the HBM budget (evicting idle problems) and refuses a
   problem larger than the budget.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -174,3 +176,28 @@ def test_a_wider_batch_keeps_its_own_slot():
     assert st["completed"] == 2 + len(freqs) and st["peak_bytes"] <= 2.5 * one
     for (d0, t0), (d1, t1) in zip(want, got):
         assert rel(d1, d0) < TOL and rel(t1, t0) < TOL
+
+
+def test_a_sweep_starts_beside_a_large_solve():
+    """While one large solve runs, a queued sweep of another mesh does not wait
+    for the whole in-flight limit to be free: at least one lockstep batch of it
+    (half of the limit) starts before the large solve is done."""
+    big, m = meshgen.config_mesh("c3_8640")[0], _mesh(27, 26, 8)
+    srv = serve.Server(form="mixed", refine=2)
+    mb, ms = srv.add_mesh(big), srv.add_mesh(m)
+    bc, kode = _bc(m, 0.0, 0.0, 1.0)
+    freqs = np.linspace(0.4, 6.0, 24)
+    bcb, kodeb = _bc(big, 0.0, 0.0, 1.2)
+    best = 0
+    for k in range(4):  # the first rounds also make the slots' buffers
+        rid = srv.submit(mb, MAT, 1.0 + k, bcb, kodeb)
+        tb = time.perf_counter()
+        ids, ts = [], []
+        for f in freqs:
+            ids.append(srv.submit(ms, MAT, float(f) + 0.01 * k, bc, kode))
+            ts.append(time.perf_counter())
+        start = [t + srv.wait(i)[2]["queue_ms"] * 1e-3 for i, t in zip(ids, ts)]
+        done = tb + srv.wait(rid)[2]["latency_ms"] * 1e-3
+        best = max(best, sum(s < done for s in start))
+    srv.close()
+    assert best >= 8
