@@ -20,6 +20,8 @@ constexpr int kMaxNpg = 8;
 constexpr int kMaxBatch = 64;
 // Largest number of iterative-refinement steps of the mixed form.
 constexpr int kMaxRefine = 8;
+// Stream priority level (steps below the highest) that means the lowest.
+constexpr int kLowestLevel = 1 << 16;
 
 // Device buffers of bem_sweep (per batch of problems).
 struct SweepBuf {
@@ -170,6 +172,7 @@ struct bem_ctx {
   int device = 0;
   int num_sms = 0;
   cudaStream_t own_stream = nullptr;
+  int own_level = bem::kLowestLevel;  // its priority, in steps below the highest
   cudaStream_t stream = nullptr;
   std::mutex mu;
   std::string last_error;
@@ -415,6 +418,9 @@ int measure_fma_peaks(bem_ctx* ctx, double* fp64_tflops, double* fp32_tflops);
 int measure_tf32_peak(bem_ctx* ctx, int n, double* tflops);
 
 int check_status(bem_ctx* ctx);
+// A context's own stream replaced by one whose priority is `level` below the
+// highest (the lowest there is, at most).
+int own_stream_priority(bem_ctx* ctx, int level);
 // The failure-path self-test kernel (bem_wait_selftest), lu.cu.
 int wait_selftest(bem_ctx* ctx, int which);
 

@@ -430,17 +430,7 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // equal priorities: 96 meshes of n = 72..1800 17.6 ms against 17.2, 40 of
 // 180..900 3.98 / 3.48, 12 of 90..1500 5.08 / 4.45, plain form, 48 of 90..1200
 // 7.79 / 6.90.
-int worker_priority(bem_ctx* w, int i) {
-  int lo = 0, hi = 0;
-  cudaStream_t s = nullptr;
-  BEM_CUDA(w, cudaDeviceGetStreamPriorityRange(&lo, &hi));
-  BEM_CUDA(w, cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, std::min(lo, hi + i)));
-  const cudaError_t e = cudaStreamSynchronize(w->own_stream);  // its allocations
-  cudaStreamDestroy(w->own_stream);
-  w->own_stream = w->stream = s;
-  BEM_CUDA(w, e);
-  return BEM_OK;
-}
+int worker_priority(bem_ctx* w, int i) { return own_stream_priority(w, i); }
 
 }  // namespace
 

@@ -120,7 +120,10 @@ typedef struct bem_ctx bem_ctx;
 int bem_ctx_create(int device, bem_ctx **out);
 int bem_ctx_destroy(bem_ctx *ctx);
 /* Runs every kernel of ctx on `stream` (a cudaStream_t); NULL restores the
- * context's own stream. */
+ * context's own stream, whose priority follows the mesh: the smaller its
+ * system, the higher, so that its solves are not held up by another context's
+ * large one.  A caller that runs several contexts on streams of its own may
+ * give them priorities the same way. */
 int bem_ctx_set_stream(bem_ctx *ctx, void *stream);
 /* Algorithm switches of a context (1 on, 0 off), for comparison and for the
  * autotuner: "tcgen05" (FP32 trailing update on tcgen05, else TF32

@@ -201,3 +201,26 @@ def test_a_sweep_starts_beside_a_large_solve():
         best = max(best, sum(s < done for s in start))
     srv.close()
     assert best >= 8
+
+
+def test_small_solves_beside_a_large_one():
+    """FP64 solves of a small mesh while the server runs one of 25920 unknowns
+    take a few times what they take alone: their panels, which need whole SMs,
+    do not wait behind the large system's updates.  (12 to 14 ms against 8
+    alone with the small context's stream at a higher priority, 60 to 160 with
+    equal ones.)"""
+    big, m = meshgen.config_mesh("c3_8640")[0], _mesh(30, 30, 9)
+    srv = serve.Server(form="plain")
+    mb, ms = srv.add_mesh(big), srv.add_mesh(m)
+    bcb, kodeb = _bc(big, 0.0, 0.0, 1.2)
+
+    def small(k):
+        return srv.wait(srv.submit(ms, MAT, 1.0 + 0.01 * k, *_bc(m, 0.01 * k, 0.0, 1.2)))[2]["latency_ms"]
+
+    srv.wait(srv.submit(mb, MAT, 0.8, bcb, kodeb))
+    alone = sorted(small(k) for k in range(5))[2]
+    rid = srv.submit(mb, MAT, 1.7, bcb, kodeb)
+    beside = sorted(small(10 + k) for k in range(5))[2]
+    assert srv.wait(rid)[2]["latency_ms"] > 5 * 3 * alone  # it ran meanwhile
+    srv.close()
+    assert beside < 4 * alone
