@@ -4101,6 +4101,31 @@ bool make_rows_map(CUtensorMap* m, const void* base, int nn, size_t lda, size_t 
 // memory would not fit, and k_trsv runs instead.
 constexpr size_t kTrsvF32SmemMax = 200 * 1024;
 
+// A table of the FP32 solves, grown to `bytes`; false when there is no memory
+// for it, and in a capture that would have to allocate it (a graph's own
+// allocation would not outlive the graph's next launch), so that a captured
+// step takes the kernel the step before it took.
+template <typename T>
+static bool solve_table(bem_ctx* ctx, T*& p, size_t& cap, size_t bytes) {
+  if (cap >= bytes) return true;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  if constexpr (std::is_same<T, float2>::value) ctx->lu.tinv_valid = ctx->lu.uinv_valid = false;  // tinv's contents go
+  dev_free(ctx, p);
+  p = nullptr;
+  cap = 0;
+  if (dev_alloc(ctx, &p, bytes) != cudaSuccess) {
+    p = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+  cap = bytes;
+  return true;
+}
+
 // The cluster form (k_trsv_cl): done = false when the factorisation's panels
 // are not 64 wide, or a CTA's rows, the permutation's tables or a ring of two
 // stages do not fit shared memory, and for systems so tall that a cluster's
@@ -4129,22 +4154,12 @@ static int trsv_cl(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, in
   const int stages = (int)std::min<size_t>(6, (kSmem - fixed) / stage);
   CUtensorMap tm;
   if (!make_rows_map(&tm, A, nn, lda, bstride, batch, 64)) return BEM_OK;
-  // (no memory for this form's tables: the cooperative kernels, which need less)
-  auto need = [&](auto*& p, size_t& cap, size_t bytes) {
-    if (cap >= bytes) return true;
-    dev_free(ctx, p);
-    p = nullptr;
-    cap = 0;
-    if (dev_alloc(ctx, &p, bytes) != cudaSuccess) {
-      p = nullptr;
-      cudaGetLastError();
-      return false;
-    }
-    cap = bytes;
-    return true;
-  };
-  if (L.tinv_bytes < (size_t)batch * (npan + nb) * stage) L.tinv_valid = L.uinv_valid = false;
-  if (!need(L.tinv, L.tinv_bytes, (size_t)batch * (npan + nb) * stage)) return BEM_OK;
+  // both tables before any kernel; without the memory for them the cooperative
+  // kernels, of which k_trsv needs neither
+  if (!solve_table(ctx, L.tinv, L.tinv_bytes, (size_t)batch * (npan + nb) * stage)) return BEM_OK;
+  if (forward && !L.lperm_valid &&
+      !solve_table(ctx, L.rmap, L.rmap_bytes, ((size_t)(npan + 1) * nn + npan) * batch * sizeof(int)))
+    return BEM_OK;
   float2* A2 = static_cast<float2*>(A);
   constexpr size_t kInvSmem = 2 * kLtTile;
   BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_tri_inv_cl), kInvSmem));
@@ -4161,7 +4176,6 @@ static int trsv_cl(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, in
     L.tinv_valid = false;
   }
   if (forward && !L.lperm_valid) {
-    if (!need(L.rmap, L.rmap_bytes, ((size_t)(npan + 1) * nn + npan) * batch * sizeof(int))) return BEM_OK;
     int* moved = L.rmap + (size_t)(npan + 1) * nn * batch;
     const size_t msm = (size_t)2 * nn * sizeof(int), psm = (size_t)nn * sizeof(float2);
     BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_row_maps), msm));
@@ -4241,13 +4255,7 @@ static int trsv_f32(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, int
   if (!group) return BEM_OK;
   if (!L.tinv_valid) {
     const size_t bytes = (size_t)batch * (npan + nblk) * kTrsvBlk * kTrsvBlk * sizeof(float2);
-    if (L.tinv_bytes < bytes) {
-      dev_free(ctx, L.tinv);
-      L.tinv = nullptr;
-      L.tinv_bytes = 0;
-      BEM_CUDA(ctx, dev_alloc(ctx, &L.tinv, bytes));
-      L.tinv_bytes = bytes;
-    }
+    if (!solve_table(ctx, L.tinv, L.tinv_bytes, bytes)) return BEM_OK;  // k_trsv instead
     ProfScope ps(ctx, 4, 8.0 * (double)(npan + nblk) * kTrsvBlk * kTrsvBlk * kTrsvBlk / 3.0 * batch,
                  2.0 * (double)(npan + nblk) * kTrsvBlk * kTrsvBlk * sizeof(float2) * batch);
     constexpr size_t kInvSmem = (size_t)2 * 64 * 65 * sizeof(float2);

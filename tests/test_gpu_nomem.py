@@ -98,3 +98,36 @@ def test_first_calls_of_a_mesh(nx, ny):
         assert count > 5
     finally:
         ctx.close()
+
+
+# 189 unknowns: one forward step of three, 720: twelve; one refinement step:
+# the solves' tables are asked for once per step
+@pytest.mark.parametrize("nx,ny", [(9, 7), (16, 15)])
+@pytest.mark.parametrize("refine", [1, 3])
+def test_mixed_sweep_and_its_captured_step(nx, ny, refine):
+    """A failure in the step that runs directly, then the captured step and its
+    replays: the solutions stay those of the plain form (to the refinement's
+    1e-6 after one step)."""
+    m, d = _mesh(nx, ny)
+    freqs = [1.0, 2.5, 4.0]
+    with _solver(m, d) as sol:
+        want, _ = sol.sweep(freqs, form="plain", batch=3)
+    tol = 1e-6 if refine == 1 else 1e-9
+    n = done = 0
+    while True:
+        n += 1
+        with _solver(m, d) as sol:
+            sol.ctx.set_option("fail_alloc", n)
+            try:
+                x, _ = sol.sweep(freqs, form="mixed", batch=3, refine=refine)
+                assert rel(x, want) < tol, n
+                done += 1
+            except capi.BemError as e:
+                assert e.code == capi.BEM_ERR_NOMEM, (n, e)
+            left = sol.ctx.get_option("fail_alloc")
+            if left:
+                break
+            for _ in range(4):  # directly or captured, then replayed
+                x, _ = sol.sweep(freqs, form="mixed", batch=3, refine=refine)
+                assert rel(x, want) < tol, n
+    assert n > 10 and done >= 2  # the solves' tables, at least, are done without
