@@ -247,6 +247,21 @@ int sweep(bem_ctx* ctx, const double zge[2], const double zcs[2], const double z
   if (rc) return rc;
   SweepBuf& S = ctx->sweep;
   const int nn = S.nn;
+  // The step's other buffers (interchange lists, tensor-core operands, solves)
+  // grow while it is enqueued: without memory for them the same step runs
+  // again with half as many problems, whose systems leave more of it.
+  auto fewer = [&]() -> int {
+    BEM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    release_sweep_graph(ctx);
+    tc_release(ctx);
+    int r;
+    do {
+      batch = (batch + 1) / 2;
+      free_sweep(ctx, S);
+      r = ensure_sweep(ctx, batch, mixed);
+    } while (r == BEM_ERR_NOMEM && batch > 1);
+    return r;
+  };
   BEM_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, ST_COUNT * sizeof(int), ctx->stream));
   std::vector<unsigned long long> hnorm;
   // One lockstep step: assembly, LU (+ refinement) of `bsz` problems.
@@ -265,8 +280,8 @@ int sweep(bem_ctx* ctx, const double zge[2], const double zcs[2], const double z
     }
     return lu_factor_solve_batch(ctx, S.A64, S.lda, S.a_stride, nn, bsz, false);
   };
-  for (int f0 = 0; f0 < nfreq; f0 += batch) {
-    const int bsz = std::min(batch, nfreq - f0);
+  for (int f0 = 0, bsz = 0; f0 < nfreq; f0 += bsz) {
+    bsz = std::min(batch, nfreq - f0);
     DynBatch db{};
     db.zge = zge;
     db.zcs = zcs;
@@ -330,6 +345,12 @@ int sweep(bem_ctx* ctx, const double zge[2], const double zcs[2], const double z
       }
     } else {
       rc = enqueue(db, bsz);
+      if (rc == BEM_ERR_NOMEM && bsz > 1) {
+        rc = fewer();
+        if (rc) return rc;
+        bsz = 0;
+        continue;
+      }
       if (rc) return rc;
       ctx->sw_nn = nn;
       ctx->sw_bsz = bsz;

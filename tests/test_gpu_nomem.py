@@ -131,3 +131,27 @@ def test_mixed_sweep_and_its_captured_step(nx, ny, refine):
                 x, _ = sol.sweep(freqs, form="mixed", batch=3, refine=refine)
                 assert rel(x, want) < tol, n
     assert n > 10 and done >= 2  # the solves' tables, at least, are done without
+
+
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+@pytest.mark.parametrize("nx,ny,count", [(9, 7, 5), (16, 15, 2)])
+def test_sweep_goes_on_with_fewer_problems(form, nx, ny, count):
+    """Whichever buffer of a lockstep step finds no memory, the sweep runs in
+    smaller steps and gives every solution."""
+    m, d = _mesh(nx, ny)
+    freqs = np.linspace(1.0, 4.0, count)
+    with _solver(m, d) as sol:
+        want, _ = sol.sweep(freqs, form="plain", batch=count)
+    n = 0
+    while True:
+        n += 1
+        with _solver(m, d) as sol:
+            sol.ctx.set_option("fail_alloc", n)
+            x, corr = sol.sweep(freqs, form=form, batch=count, refine=3)
+            assert rel(x, want) < 1e-9 and np.all(corr < 1e-7), n
+            left = sol.ctx.get_option("fail_alloc")
+            if left:
+                break
+            x, _ = sol.sweep(freqs, form=form, batch=count, refine=3)
+            assert rel(x, want) < 1e-9, n
+    assert n > 10
