@@ -457,12 +457,11 @@ int worker_priority(bem_ctx* w, int i) { return own_stream_priority(w, i); }
 
 constexpr int kBatchWorkers = 8;
 
-int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freqs, const double* zge,
-                const double* zcs, const double* zcp, const double* c, int form, int iters, double* const* x_out,
-                double* corr_out) {
-  const bool mixed = form == BEM_FORM_MIXED;
-  if (!mixed && form != BEM_FORM_PLAIN) return fail(d, BEM_ERR_ARG, "unknown form");
-  if (iters < 0 || iters > kMaxRefine) return fail(d, BEM_ERR_ARG, "refinement steps out of range");
+// One pass over all problems, in classes of at most `limit`; widest: the
+// largest class.
+static int batch_pass(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freqs, const double* zge,
+                      const double* zcs, const double* zcp, const double* c, bool mixed, int iters,
+                      double* const* x_out, double* corr_out, int limit, int* widest) {
   std::vector<int> order(nprob);
   for (int i = 0; i < nprob; ++i) order[i] = i;
   std::sort(order.begin(), order.end(), [&](int a, int b) { return probs[a]->mesh.nbe < probs[b]->mesh.nbe; });
@@ -496,7 +495,7 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
     while (g1 < nprob) {
       const int n1 = 3 * probs[order[g1]]->mesh.nbe;
       if (n1 * 4 > n0 * 5) break;
-      if (g1 - g0 + 1 > std::min(kMaxBatch, lu_lockstep_capacity(d, n1, mixed))) break;
+      if (g1 - g0 + 1 > std::min(limit, lu_lockstep_capacity(d, n1, mixed))) break;
       npad = n1;
       ++g1;
     }
@@ -505,6 +504,7 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
       diag += (size_t)9 * probs[order[k]]->mesh.nbe;
       rhs += (size_t)rhs_chunks(probs[order[k]]) * 3 * probs[order[k]]->mesh.nbe;
     }
+    *widest = std::max(*widest, g1 - g0);
     plan.push_back({g0, g1, npad, sol_total, diag, rhs});
     sol_total += (size_t)(g1 - g0) * npad;
     g0 = g1;
@@ -654,6 +654,32 @@ int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freq
     }
   }
   return BEM_OK;
+}
+
+// Without memory for some class, all of it once more in classes half as wide:
+// the lockstep limit allows more than the device may hold (eight workers, up
+// to 18 problems of 6480 unknowns each, 19 GB a class).
+int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freqs, const double* zge,
+                const double* zcs, const double* zcp, const double* c, int form, int iters, double* const* x_out,
+                double* corr_out) {
+  const bool mixed = form == BEM_FORM_MIXED;
+  if (!mixed && form != BEM_FORM_PLAIN) return fail(d, BEM_ERR_ARG, "unknown form");
+  if (iters < 0 || iters > kMaxRefine) return fail(d, BEM_ERR_ARG, "refinement steps out of range");
+  for (int limit = kMaxBatch;;) {
+    int widest = 0;
+    const int rc =
+        batch_pass(d, nprob, probs, freqs, zge, zcs, zcp, c, mixed, iters, x_out, corr_out, limit, &widest);
+    if (rc == BEM_OK) return rc;
+    // nothing of a pass that failed is left running: its staging is reused
+    for (bem_ctx* w : d->workers) cudaStreamSynchronize(w->stream);
+    if (rc != BEM_ERR_NOMEM || widest <= 1) return rc;
+    for (bem_ctx* w : d->workers) {
+      free_sweep(w, w->bbuf);
+      tc_release(w);
+      cudaStreamSynchronize(w->stream);  // the next worker's allocation may take it
+    }
+    limit = (widest + 1) / 2;
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -155,3 +155,40 @@ def test_sweep_goes_on_with_fewer_problems(form, nx, ny, count):
             x, _ = sol.sweep(freqs, form=form, batch=count, refine=3)
             assert rel(x, want) < 1e-9, n
     assert n > 10
+
+
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+def test_batch_goes_on_in_smaller_classes(form):
+    """Whichever allocation of a batch call fails, on the driver or a worker,
+    the call gives every solution; so does the next one."""
+    from bem_mececcs_b200.solver import batch_solve
+    probs = []
+    want = []
+    for k, (nx, ny) in enumerate([(3, 2), (9, 7), (9, 7), (9, 8), (10, 7), (16, 15)]):
+        sol = _solver(*_mesh(nx, ny))
+        fr = 1.0 + 0.3 * k
+        want.append(sol.sweep([fr], form="plain", batch=1)[0][0])
+        probs.append((sol, fr))
+    n = ok = 0
+    while True:
+        n += 1
+        ctx = capi.Context(0)
+        try:
+            ctx.set_option("fail_alloc", n)
+            try:
+                xs, _ = batch_solve(ctx, probs, form=form, refine=3)
+                assert all(rel(x, w) < 1e-9 for x, w in zip(xs, want)), n
+                ok += 1
+            except capi.BemError as e:  # a class of one problem has nothing to give up
+                assert e.code == capi.BEM_ERR_NOMEM, (n, e)
+            left = ctx.get_option("fail_alloc")
+            ctx.set_option("fail_alloc", 0)
+            xs, _ = batch_solve(ctx, probs, form=form, refine=3)
+            assert all(rel(x, w) < 1e-9 for x, w in zip(xs, want)), n
+        finally:
+            ctx.close()
+        if left:
+            break
+    for sol, _ in probs:
+        sol.close()
+    assert n > 20 and ok == n
