@@ -89,6 +89,7 @@ def lib():
     L.bem_measure_fp64_peak.argtypes = [vp, vp]
     L.bem_measure_peaks.argtypes = [vp, vp]
     L.bem_wait_selftest.argtypes = [vp, ip]
+    L.bem_math_selftest.argtypes = [vp, ip, ip, vp, vp]
     L.bem_static_solve.argtypes = [vp, vp, dp, vp, vp, vp, vp]
     L.bem_batch_solve.argtypes = [vp, ip, vp, vp, vp, vp, vp, vp, ip, ip, vp, vp]
     L.bem_interior.argtypes = [vp, vp, vp, vp, dp, dp, ip, vp, vp, vp, vp, vp, vp, vp]
@@ -184,6 +185,14 @@ class Context:
         never happens (0: bulk-copy mbarrier, 1: grid barrier); BEM_ERR_TIMEOUT
         when the wait gave up as it should."""
         return int(self.L.bem_wait_selftest(self.h, int(which)))
+
+    def math_selftest(self, which: int, args) -> np.ndarray:
+        """bem_math_selftest: 0, args [n, 3] -> [n, 4]; 1, args [n] -> [n, 3]."""
+        args = f64(args)
+        out = np.zeros((len(args), 4 if which == 0 else 3))
+        self.check(self.L.bem_math_selftest(self.h, int(which), len(args), ptr(args), ptr(out)),
+                   "bem_math_selftest")
+        return out
 
     def fp64_peak_tflops(self) -> float:
         out = np.zeros(1)

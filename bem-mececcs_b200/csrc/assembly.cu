@@ -1178,3 +1178,51 @@ int bem_ghmatecd_noalloc(bem_ctx* ctx, const double zge[2], const double zcs[2],
   if (ctx->mesh_flag_bnd) return fail(ctx, BEM_ERR_DEGENERATE, "Jacobian below 1e-5 on a boundary element");
   return BEM_OK;
 }
+
+// ---------------------------------------------------------------------------
+// Self-test of the kernels' own elementary functions (cexp.cuh).
+// ---------------------------------------------------------------------------
+namespace bem {
+
+__global__ void __launch_bounds__(128) k_math_selftest(int which, int n, const double* __restrict__ in, double* out) {
+  __shared__ CexpTable tab;
+  cexp_table_fill(tab);
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if (which == 0) {
+    const double re = in[3 * i], im = in[3 * i + 1], scale = in[3 * i + 2];
+    const double2 e = cexp_tab(tab, re, im, scale, re != 0.0), g = cexp_general(re, im);
+    out[4 * i] = e.x;
+    out[4 * i + 1] = e.y;
+    out[4 * i + 2] = g.x * scale;
+    out[4 * i + 3] = g.y * scale;
+  } else {
+    out[3 * i] = rsqrt_fast(in[i]);
+    out[3 * i + 1] = rsqrt_seed(in[i]);
+    out[3 * i + 2] = rsqrt(in[i]);
+  }
+}
+
+}  // namespace bem
+
+int bem_math_selftest(bem_ctx* ctx, int which, int n, const double* in, double* out) {
+  if (!ctx || (which != 0 && which != 1) || n < 0 || n > (1 << 26) || (n > 0 && (!in || !out))) return BEM_ERR_ARG;
+  if (n == 0) return BEM_OK;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  cudaSetDevice(ctx->device);
+  const size_t ni = (size_t)n * (which == 0 ? 3 : 1), no = (size_t)n * (which == 0 ? 4 : 3);
+  double* d = nullptr;
+  BEM_CUDA(ctx, dev_alloc(ctx, &d, (ni + no) * sizeof(double)));
+  cudaError_t e = cudaMemcpyAsync(d, in, ni * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) {
+    k_math_selftest<<<(n + 127) / 128, 128, 0, ctx->stream>>>(which, n, d, d + ni);
+    ctx->launches++;
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, d + ni, no * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+  const cudaError_t es = cudaStreamSynchronize(ctx->stream);
+  dev_free(ctx, d);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? BEM_OK : cuda_fail(ctx, e, "bem_math_selftest");
+}

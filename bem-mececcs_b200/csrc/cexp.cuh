@@ -11,6 +11,13 @@
 // the general functions', which also carry the code for huge arguments.
 // Arguments outside the tables' reduction (|phase| above 1e7, |exponent|
 // above 700, not finite) take the general functions.
+//
+// Accuracy, in u = 2^-53 of the modulus (tests/test_gpu_math.py derives and
+// checks the bounds): undamped at most 2.7 (measured 2.1; the general
+// functions with the same products 1.7), damped at most 6.1 (3.5; 2.7), sines
+// below pi/128 2.1 relative, 1/sqrt at most 1.6 (1.24; CUDA's rsqrt 1.01).
+// The results built on them are no further from 64-bit values than with the
+// general functions, since the radial functions round fewer terms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -131,11 +138,15 @@ __device__ __forceinline__ double2 cexp_tab(const CexpTable& tab, double re, dou
   return make_double2(e * fma(-t.x, sr, fma(t.y, cr, t.y)), e * fma(t.y, sr, fma(t.x, cr, t.x)));
 }
 
-// 1 / sqrt(x), x > 0: the hardware's approximation (about 20 bits) refined by
-// one step of Householder's third-order iteration.
-__device__ __forceinline__ double rsqrt_fast(double x) {
+// 1 / sqrt(x), x > 0 and normal: the hardware's approximation (measured within
+// 2^-20.08) refined by one step of Householder's third-order iteration.
+__device__ __forceinline__ double rsqrt_seed(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rsqrt_fast(double x) {
+  const double y = rsqrt_seed(x);
   const double e = fma(-x * y, y, 1.0);
   return fma(y * e, fma(kCx[13], e, 0.5), y);
 }

@@ -349,6 +349,13 @@ int bem_prof_bytes(bem_ctx *ctx, double *bytes);
  * Nothing faults or hangs. */
 int bem_wait_selftest(bem_ctx *ctx, int which);
 
+/* Accuracy self-test of the kernels' own elementary functions, n arguments.
+ * which 0: in[n][3] = re, im, scale, out[n][4] = scale exp(re + i im) by the
+ * tables, then by CUDA's exp and sincos (re, im).  which 1: in[n] = x > 0
+ * (normal), out[n][3] = 1/sqrt(x) as the kernels form it, the hardware's
+ * approximation it starts from, CUDA's rsqrt. */
+int bem_math_selftest(bem_ctx *ctx, int which, int n, const double *in, double *out);
+
 /* Measures this GPU's FP64 tensor-core (DMMA) throughput with a
  * register-resident mma.sync loop; writes TFLOP/s. */
 int bem_measure_fp64_peak(bem_ctx *ctx, double *tflops);
