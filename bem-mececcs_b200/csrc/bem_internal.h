@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
+#include <map>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -80,6 +82,12 @@ struct System {
 // Gather list of one panel's row interchanges: count, then dst/src pairs.
 constexpr int kPermStride = 1 + 2 * 128;
 
+// Shape of a cooperative FP32 solve (trsv_f32_shape).
+struct TrsvShape {
+  int group = 0, ldl = 0, sub = 0;  // CTAs per problem, rows of a share's box, problems per launch (0: not worked out)
+  size_t smem = 0;
+};
+
 struct LuWork {
   int cap_nn = 0, cap_batch = 0;
   int cluster_cs = 0;           // CTAs per panel cluster (16 or 8)
@@ -114,6 +122,7 @@ struct LuWork {
   size_t ts_cap[7] = {0, 0, 0, 0, 0, 0, 0};  // elements allocated, in the order above
   float2* tinv = nullptr;        // FP32 solves: inverted diagonal blocks of the last factors
   size_t tinv_bytes = 0;
+  std::map<std::array<int, 3>, TrsvShape> trsv_shapes;  // by unknowns, problems and CTA budget
   bool tinv_valid = false;
   bool uinv_valid = false;       // k_trsv_cl: tinv holds the U blocks' inverses by columns
   bool lperm_valid = false;      // ... and the L blocks', and L is in its final row order

@@ -4222,36 +4222,65 @@ static int trsv_cl(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, in
   return BEM_OK;
 }
 
+// How k_trsv_f32 runs `batch` systems of nn unknowns: the largest group of CTAs
+// per problem (at most a CTA per SM, which a 25920-unknown system needs for its
+// shares to fit a box) that are all resident; a share is at most 256 rows (one
+// TMA box), so a large batch of large systems is solved by several launches of
+// `sub` problems.  group = 0: no shape fits.  Occupancy queries take tens of
+// microseconds and every solve asks, so a shape is worked out once per context;
+// larger shares are never more resident, which bounds the groups to try.
+static int trsv_f32_shape(bem_ctx* ctx, int nn, int batch, TrsvShape& out) {
+  TrsvShape& s = ctx->lu.trsv_shapes[{nn, batch, ctx->trsv_ctas}];
+  if (s.sub) {
+    out = s;
+    return BEM_OK;
+  }
+  TrsvShape t;
+  auto share = [&](int g) {
+    t.ldl = ((nn + g - 1) / g + 3) & ~1;  // rows of a share rounded out to even ends
+    t.smem = (size_t)kTrsvBlk * t.ldl * sizeof(float2) + (size_t)t.ldl * sizeof(int) + 128;
+    return t.smem <= kTrsvF32SmemMax && t.ldl <= 256;  // (smaller groups only need more)
+  };
+  auto slots = [&](int& n) -> int {
+    BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_trsv_f32), t.smem));
+    BEM_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_trsv_f32, 256, t.smem));
+    n *= ctx->num_sms;
+    if (ctx->trsv_ctas > 0) n = std::min(n, ctx->trsv_ctas);
+    return BEM_OK;
+  };
+  const int gmax = std::min(std::max(64, ctx->num_sms), std::max(1, (nn + kTrsvBlk - 1) / kTrsvBlk));
+  int most = 0, rc = BEM_OK;
+  if (share(gmax) && (rc = slots(most))) return rc;
+  t.sub = batch;
+  for (int parts = 1, last = 0; !t.group && parts <= batch; ++parts) {
+    t.sub = (batch + parts - 1) / parts;
+    if (t.sub == last) continue;
+    last = t.sub;
+    for (int g = std::min(gmax, most / t.sub); g >= 1 && share(g); --g) {
+      int n = 0;
+      rc = slots(n);
+      if (rc) return rc;
+      if (g * t.sub <= n) {
+        t.group = g;
+        break;
+      }
+    }
+  }
+  out = s = t;
+  return BEM_OK;
+}
+
 static int trsv_f32(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, int nn, int batch, void* v,
                     size_t vstride, bool forward, bool& done) {
   LuWork& L = ctx->lu;
   done = false;
   const int npan = (int)L.panels.size(), nblk = (nn + kTrsvBlk - 1) / kTrsvBlk;
-  // The largest group (at most a CTA per SM, which a 25920-unknown system needs
-  // for its shares to fit a box) whose CTAs are all resident; a share is at most 256 rows (one TMA box), so a large batch of
-  // large systems is solved by several launches of fewer problems.
-  int group = 0, ldl = 0, sub = batch;
-  size_t smem = 0;
-  for (int parts = 1; !group && parts <= batch; ++parts) {
-    sub = (batch + parts - 1) / parts;
-    for (int g = std::min(std::max(64, ctx->num_sms), std::max(1, nblk)); g >= 1; --g) {
-      const int per = (nn + g - 1) / g;
-      const int l = (per + 3) & ~1;  // rows of a share rounded out to even ends
-      const size_t sm = (size_t)kTrsvBlk * l * sizeof(float2) + (size_t)l * sizeof(int) + 128;
-      if (sm > kTrsvF32SmemMax || l > 256) break;  // smaller groups only need more; TMA boxes <= 256 rows
-      BEM_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(k_trsv_f32), sm));
-      int occ = 0;
-      BEM_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trsv_f32, 256, sm));
-      int slots = occ * ctx->num_sms;
-      if (ctx->trsv_ctas > 0) slots = std::min(slots, ctx->trsv_ctas);
-      if (g * sub <= slots) {
-        group = g;
-        ldl = l;
-        smem = sm;
-        break;
-      }
-    }
-  }
+  TrsvShape shape;
+  const int src = trsv_f32_shape(ctx, nn, batch, shape);
+  if (src) return src;
+  const int group = shape.group, sub = shape.sub;
+  int ldl = shape.ldl;
+  const size_t smem = shape.smem;
   if (!group) return BEM_OK;
   if (!L.tinv_valid) {
     const size_t bytes = (size_t)batch * (npan + nblk) * kTrsvBlk * kTrsvBlk * sizeof(float2);
