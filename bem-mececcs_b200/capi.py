@@ -142,7 +142,7 @@ class Context:
         except Exception:
             pass
 
-    INT_OPTIONS = ("gemm_ctas", "trsv_ctas", "wait_limit_ms", "fail_alloc")
+    INT_OPTIONS = ("gemm_ctas", "trsv_ctas", "wait_limit_ms", "fail_alloc", "lookahead_runs")
 
     def set_option(self, name: str, value) -> None:
         """bem_ctx_set_option: switches tcgen05, trsv_coop, lu_pairs, lu_quads,

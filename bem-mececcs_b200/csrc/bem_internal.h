@@ -237,6 +237,7 @@ struct bem_ctx {
   cudaEvent_t crit_ev[3] = {nullptr, nullptr, nullptr};
   void* crit_ws = nullptr;    // cuBLAS workspace of its products
   bool lu_lookahead = true;   // LU: panels run beside the previous group's update
+  int lookahead_runs = 0;     // factorisations enqueued (or captured) that way
   int panel_share = 1;        // LU: panels to size for running at the same time (bem_batch_solve's workers)
   bool panel_calu = false;    // FP32 LU panels: tournament pivoting per 8-column sub-panel
   bool panel_push = true;     // cluster panels exchange pivots by remote stores before the barrier

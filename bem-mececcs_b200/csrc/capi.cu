@@ -716,6 +716,10 @@ int bem_ctx_get_option(bem_ctx* ctx, const char* name, int* value) {
     *value = ctx->wait_limit_ms;
     return BEM_OK;
   }
+  if (!strcmp(name, "lookahead_runs")) {  // read only
+    *value = ctx->lookahead_runs;
+    return BEM_OK;
+  }
   if (bool* slot = option_slot(ctx, name)) {
     *value = *slot ? 1 : 0;
     return BEM_OK;

@@ -4402,7 +4402,13 @@ static int trsv_coop(bem_ctx* ctx, const void* A, size_t lda, size_t bstride, in
 //   main:  each panel's interchanges of [kG, ncols) as it is done
 //          (main_waits), the last one's of [kN, ncols) only; the update of
 //          [kN, ncols).
-// Every column takes the same operations in the same order as without it.
+// An FP32 column takes the same operations in the same order as without it.
+// In FP64 the pair's update is two ZGEMMs of other widths, so results may
+// differ at rounding level with lookahead on or off; it is off below the
+// sizes of lookahead_shape, with other than the default kernels, while kernel
+// classes are timed, under a CTA budget, in a capture whose buffers are not
+// there yet, in the server's slots and the workers of a batch call, and where
+// free memory is short (lookahead_room).
 struct Lookahead {
   bem_ctx* ctx;
   cudaStream_t main;
@@ -4806,6 +4812,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
   if (look) {
     int rc = la.fork();
     if (rc) return rc;
+    ctx->lookahead_runs++;
   }
   for (int k = 0; k < nn;) {
     const int m = nn - k;

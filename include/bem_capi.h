@@ -146,7 +146,10 @@ int bem_ctx_set_stream(bem_ctx *ctx, void *stream);
  * mbarrier-counted mailboxes, without a cluster barrier per column),
  * "lu_lookahead" (large factorisations: panels on a second, high-priority
  * stream beside the previous update; the call's work still begins and ends on
- * the context's stream), "laswp_tc" (FP32 row interchanges + U12 on the tensor
+ * the context's stream; FP32 factors are the same with and without, FP64
+ * results agree to rounding; not used where free memory is short or kernel
+ * classes are timed; "lookahead_runs", read only, counts the factorisations
+ * enqueued that way), "laswp_tc" (FP32 row interchanges + U12 on the tensor
  * cores), "trsv_inv"
  * (FP32 solves with inverted diagonal blocks), "graphs" (bem_sweep replays a
  * captured step).  Defaults: tcgen05, tc_pair, trsv_coop, lu_pairs,

@@ -57,3 +57,45 @@ def test_sweep(form, nx, ny, batch):
                 assert np.array_equal(x[1][i], x[0][i]), freqs[i]
             else:
                 assert rel(x[1][i], x[0][i]) < 1e-11, freqs[i]
+
+
+# the cases above, which lie just over the rule's lines, and one below each
+@pytest.mark.parametrize("form,nx,ny,batch,used", [
+    ("plain", 10, 9, 35, True), ("plain", 13, 10, 17, True), ("plain", 17, 10, 10, True), ("plain", 25, 19, 2, True),
+    ("mixed", 25, 19, 13, True), ("mixed", 20, 17, 25, True), ("mixed", 43, 10, 16, True),
+    ("mixed", 29, 33, 4, True), ("plain", 10, 9, 34, False), ("mixed", 25, 19, 12, False)])
+def test_lookahead_is_used(form, nx, ny, batch, used):
+    """The comparisons above say something only where lookahead runs with the
+    option on, and does not with it off."""
+    m = meshgen.enclosed_grid(nx, ny, jitter=0.10, seed=3, depth=2.5, layers=2)
+    d = meshgen.traction_patch(m, radius=6.0, dam=0.02)
+    with BemSolver(m) as sol:
+        sol.ghmatece()
+        sol.set_bc(d.kode, d.bc, d.dam, d.rho)
+        freqs = np.linspace(3.0, 14.0, batch)
+        for on in (1, 0):
+            sol.ctx.set_option("lu_lookahead", on)
+            before = sol.ctx.get_option("lookahead_runs")
+            for _ in range(2):  # enqueued directly, then captured where it can be
+                sol.sweep(freqs, form=form, batch=batch, refine=1)
+            runs = sol.ctx.get_option("lookahead_runs") - before
+            assert runs >= 2 if used and on else runs == 0
+
+
+@pytest.mark.parametrize("n,used", [(1581, False), (1582, True), (2241, True)])
+def test_lookahead_is_used_by_one_system(n, used):
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    b = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    x = {}
+    for on in (1, 0):
+        ctx = capi.Context(0)
+        try:
+            ctx.set_option("lu_lookahead", on)
+            x[on] = solve_dense(ctx, a, b)
+            assert ctx.get_option("lookahead_runs") == (1 if used and on else 0)
+        finally:
+            ctx.close()
+    # two backward-stable solves of one system: apart by its condition, which
+    # for these matrices is below n^2
+    assert rel(x[1], x[0]) < 10 * n ** 2 * np.finfo(float).eps
