@@ -4534,14 +4534,21 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
   // FP32 (the mixed form) pivots by tournament per 8-column sub-panel.
   const bool calu = sizeof(R) == 4 && ctx->panel_calu;
   const bool ip = panel_ip_on(ctx, sizeof(R) == 4);
-  auto panel_nb = [&](int m) {
-    if (ip && panel_shape<R>(ctx, m, batch).cs) return 64;
+  auto cluster_nb = [&](int m) {
     const int rp_c = (m + cs - 1) / cs;
     if (rp_c <= 512)
       for (int cand : {64, 32, 16})
         if (calu ? calu_panel_fits_any(cand, rp_c) : cluster_panel_fits_any<R>(cand, rp_c)) return cand;
     return 0;
   };
+  // k_panel_ip's shape; none when it is off or too short for the panel, nor for
+  // panels that the option panel_tslu asks a tournament for (FP32, too tall for
+  // the other cluster kernels)
+  auto ip_shape = [&](int m) {
+    if (!ip || (sizeof(R) == 4 && ctx->panel_tslu && cluster_nb(m) == 0)) return PanelShape{};
+    return panel_shape<R>(ctx, m, batch);
+  };
+  auto panel_nb = [&](int m) { return ip_shape(m).cs ? 64 : cluster_nb(m); };
   // Factors the panel starting at column k; returns its width and gather lists.
   auto run_panel = [&](int k, int& w, int*& perm_p) -> int {
     const int m = nn - k;
@@ -4562,7 +4569,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
     pa.async_mail = ctx->panel_async ? 1 : 0;
     const int nb = panel_nb(m);
     ProfScope ps(ctx, 1, 0.0, 2.0 * (double)m * std::min(nb ? nb : 64, m) * es * batch);
-    const PanelShape sh = ip ? panel_shape<R>(ctx, m, batch) : PanelShape{};
+    const PanelShape sh = ip_shape(m);
     if (sh.cs) {
       w = std::min(64, m);
       pa.w = w;
@@ -4784,7 +4791,7 @@ static int lu_run(bem_ctx* ctx, void* A, size_t lda, size_t bstride, int nn, int
   };
   // Lookahead: the default kernels only, and not while kernel classes are
   // timed one by one or the context has only a share of the SMs.
-  bool look = ctx->lu_lookahead && !ctx->prof.on && ctx->gemm_ctas == 0 && ip &&
+  bool look = ctx->lu_lookahead && !ctx->prof.on && ctx->gemm_ctas == 0 && ip_shape(nn).cs > 0 &&
                     (sizeof(R) == 8 ? ctx->f64_pairs && ctx->f64_cublas
                                     : tc && ctx->tc_pair && ctx->lu_quads && ctx->lu_pairs && ctx->laswp_tc) &&
                     lookahead_shape<R>(ctx, nn, batch);

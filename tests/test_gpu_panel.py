@@ -79,3 +79,27 @@ def test_fp32_solves_with_interchanges(nx, ny, count):
         xm, _ = sol.sweep(freqs, form="mixed", batch=count, refine=7)
         for i in range(count):
             assert rel(xm[i], xp[i]) < 1e-9, freqs[i]
+
+
+def test_tournament_option_reaches_tall_panels():
+    """n = 8250: the first FP32 panel has more rows than the push kernel's
+    cluster holds (8192), so the option panel_tslu factors it by a tournament
+    (six launches) whatever the in-place kernel could hold.  Its candidates go
+    through k_panel_push with mailboxes.  The refined solution reaches the
+    plain form's."""
+    m = meshgen.enclosed_grid(55, 50, jitter=0.10, seed=9, depth=2.5, layers=2)
+    d = meshgen.traction_patch(m, radius=2.0)
+    launches = {}
+    with BemSolver(m) as sol:
+        sol.ghmatece()
+        sol.set_bc(d.kode, d.bc, d.dam, d.rho)
+        assert sol.nn == 8250
+        sol.ctx.set_option("lu_lookahead", 0)  # which splits launches, and is for the in-place kernel
+        xp, _ = sol.sweep([1.3], form="plain", batch=1)
+        for on in (0, 1):
+            sol.ctx.set_option("panel_tslu", on)
+            before = sol.ctx.launches
+            xm, _ = sol.sweep([1.3], form="mixed", batch=1, refine=3)
+            launches[on] = sol.ctx.launches - before
+            assert rel(xm[0], xp[0]) < 1e-10, on
+    assert launches[1] == launches[0] + 5
