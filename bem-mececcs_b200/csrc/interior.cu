@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kIntThreads) k_interior(InteriorParams p) {
         }
     }
   }
-  // CTA reduction in a fixed order: warp tree, then the 4 warps in order.
+  // CTA reduction in a fixed order: warp tree, then the warps in order.
 #pragma unroll
   for (int i = 0; i < kIntAcc; ++i) {
 #pragma unroll

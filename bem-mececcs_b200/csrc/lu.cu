@@ -6,28 +6,39 @@
 // nn, so the forward substitution happens during the factorisation.  A batch
 // of B equal-size problems (A_b = A + b * bstride) is factored in lockstep.
 //
-//   for each panel of w columns starting at k (w adapts to the panel height):
-//     k_panel_push     one thread-block cluster (16 CTAs) per problem holds the
-//                      panel rows in shared memory; per column every CTA pushes
-//                      its pivot candidate (and the owner row gj) into mailboxes
-//                      in every CTA (st.async, counted by an mbarrier).  Pivot =
-//                      first row of largest |re|+|im| (LAPACK IZAMAX); rows are
-//                      interchanged as ZGETF2 does.  k_panel_cluster (pull form)
-//                      and k_panel_calu (tournament pivoting) are options.
-//     k_panel_grid     fallback for panels too tall for one cluster: the same
-//                      algorithm over a cooperative grid with a bounded
-//                      software grid barrier.
-//     k_l11_inv +      FP32: L11^-1 once per panel, then the panel's row
-//     k_laswp_tc       interchanges on every column to the right and U12 =
-//                      L11^-1 A12 on TF32 tensor cores (with the deferred update
-//                      of the earlier panels of a group); k_laswp_trsm does the
-//                      same by substitution (FP64).
-//     k_gemm_f64       A22 -= L21 U12 on the FP64 tensor cores (DMMA m8n8k4).
-//     k_gemm_tc        (gemm_tc.cu) the FP32 update on tcgen05, K = 64 G for a
-//                      group of G = 1, 2 or 4 panels; k_gemm_tf32 on mma.sync.
-//   k_trsv_f32 /       forward + back substitution in one cooperative launch
-//   k_trsv             (FP32 with inverted diagonal blocks from k_tri_inv;
-//                      FP64 by substitution); k_backsub per 64-row block.
+//   for each panel of w columns starting at k (64 with the default kernels):
+//     k_panel_ip       (panel.cuh, default) one thread-block cluster of 1 to 16
+//                      CTAs per problem; rows stay in place until the panel is
+//                      written, pivot candidates go to every CTA's mailbox by
+//                      st.async.  Pivot = first row of largest |re|+|im| (LAPACK
+//                      IZAMAX).  Options: k_panel_push (candidates and row gj as
+//                      remote stores, rows interchanged as ZGETF2 does),
+//                      k_panel_cluster (pull form), k_panel_calu (tournament per
+//                      sub-panel), k_tslu_* (tournament over chunks of rows).
+//     k_panel_grid     panels too tall for a cluster (above 32768 FP32 or 8192
+//                      FP64 rows): the same algorithm over a cooperative grid
+//                      with a bounded software grid barrier.
+//     k_l11_inv +      FP32: L11^-1 and the group's earlier L as fragments once
+//     k_laswp_tc       per panel, then the panel's row interchanges on every
+//                      column to the right and U12 = L11^-1 A12 on TF32 tensor
+//                      cores (with the deferred update of the earlier panels of
+//                      a group); k_laswp_trsm does the same by substitution
+//                      (option laswp_tc off).
+//     k_laswp_f64      FP64: interchanges and U12 on DMMA tiles.
+//     ZGEMM            FP64: A22 -= L21 U12 by cuBLAS, two panels per update
+//                      (k_gather_l_pair); option f64_cublas off: k_gemm_f64.
+//     k_gemm_tc2       (gemm_tc.cu) the FP32 update on tcgen05 by CTA pairs, K =
+//                      64 G for a group of G = 1, 2 or 4 panels; options
+//                      k_gemm_tc (single CTAs), k_gemm_tf32 (mma.sync).
+//   Large factorisations run the panels, and what the next panels need, on a
+//   stream of the highest priority beside the previous update (Lookahead).
+//   k_trsv_cl          (trsv.cuh) FP32 solves: L in its final row order, one
+//                      cluster per problem; k_trsv_f32 (one cooperative launch,
+//                      inverted diagonal blocks) for taller systems and under a
+//                      CTA budget.
+//   k_trsv             FP64 solves in one cooperative launch, and FP32 ones
+//                      where there is no memory for the others' tables;
+//                      k_backsub per 64-row block (option trsv_coop off).
 //
 // Row interchanges are never applied to columns left of a panel; each panel's
 // interchanges are kept (ipiv and a dst/src gather list) so that later solves
@@ -624,7 +635,8 @@ __device__ __forceinline__ T sel(const T (&x)[N], int j) {
 
 // ---------------------------------------------------------------------------
 // Panel factorisation in one thread-block cluster per problem, push form
-// (the default).  Same partition as k_panel_cluster: CTA `rank` owns panel
+// (option panel_async off; with the mailboxes of async_mail in the rounds of
+// a tall panel's tournament, option panel_tslu).  Same partition as k_panel_cluster: CTA `rank` owns panel
 // rows [k + rank*rp, ...) in shared memory, one row per thread, and the
 // panel advances in 8-column sub-panels held in registers.  Every transfer
 // of a column step is a remote STORE issued before the cluster barrier:
@@ -3721,9 +3733,13 @@ static int panel_slice(int rp) {
 // factors do not depend on how many problems run together).  FP32: up to 416
 // rows per CTA, one 64-column slice, while 8 CTAs do (n <= 3328: 102 us for a
 // panel of 2871 rows against 140 in slices of 32 on 4 CTAs); then 8 CTAs up to
-// 832 rows each (slices of 32: 148 us at 6480 rows, but 16 problems at a time,
-// where 16-CTA clusters take 117 us for 7), then 16.  FP64: up to 200 rows
-// (one slice) while 8 CTAs do, then up to 256, then 16 CTAs.
+// 832 rows each, which is slices of 64 to 3344 rows, 48 to 4112, 40 to 5136,
+// 32 to 6544 and 24 to 6656 (148 us at 6480 rows, but 15 to 18 problems at a time,
+// where 16-CTA clusters take 117 us for 7); then 16 CTAs, one slice to 6688 rows,
+// then 48, 40, 32, 24, 16 and, above 26400, 8 columns.  FP64: up to 200 rows
+// while 8 CTAs do (one slice up to 194 rows, 48 columns above), then up to 256
+// (48 columns to 1680 rows, then 40), then 16 CTAs (64 columns to 3104 rows, 48
+// to 3360, 40 to 4384, 32 to 5920, 24 to 7968, then 16).
 template <typename R>
 static int panel_cs_min(int m, int cs_max) {
   int cs = 1;
@@ -3783,7 +3799,7 @@ static int launch_panel_ip_t(bem_ctx* ctx, const PanelArgs& pa, int batch) {
   return BEM_OK;
 }
 
-// Row warps and rows per thread: measured fastest at each count (eight row
+// Row warps and rows per thread for the rows a CTA has: measured fastest at each count (eight row
 // warps once two rows per thread on four would be needed, except FP64 up to
 // 256 rows).
 template <typename R>

@@ -658,7 +658,7 @@ static int batch_pass(bem_ctx* d, int nprob, bem_ctx* const* probs, const double
 
 // Without memory for some class, all of it once more in classes half as wide:
 // the lockstep limit allows more than the device may hold (eight workers, up
-// to 18 problems of 6480 unknowns each, 19 GB a class).
+// to 18 problems of 6480 unknowns each, 18 GB a class).
 int batch_solve(bem_ctx* d, int nprob, bem_ctx* const* probs, const double* freqs, const double* zge,
                 const double* zcs, const double* zcp, const double* c, int form, int iters, double* const* x_out,
                 double* corr_out) {

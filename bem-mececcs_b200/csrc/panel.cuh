@@ -3,9 +3,9 @@
 //
 // A panel of w <= 64 columns is factored by a cluster of cs CTAs, CTA `rank`
 // owning rows [k + rank * rp, ...).  Columns advance in slices of `sl` (the
-// widest of 64/32/16/8 whose rows fit shared memory) and, inside a slice, in
-// sub-panels of 8 columns whose values stay in registers (RPT rows per
-// thread of the first RW warps; the last four warps do the bookkeeping).
+// widest multiple of 8 up to 64 whose rows fit shared memory) and, inside a
+// slice, in sub-panels of 8 columns whose values stay in registers (RPT rows
+// per thread of the first RW warps; the last four warps do the bookkeeping).
 //
 // What bounds it: a chain of w pivot steps, each a reduction over all rows,
 // one exchange between the CTAs and one rank-1 update.  Measured on B200 with

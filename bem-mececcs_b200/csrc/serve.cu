@@ -37,7 +37,7 @@ using Clock = std::chrono::steady_clock;
 
 // Work in flight at once: at most 8 slots (independent solves or lockstep
 // batches) and 16 problems.  Every LU keeps one panel cluster per problem and
-// the device holds 18 8-CTA or about 9 16-CTA clusters at a time; admitting
+// the device holds 15 to 18 8-CTA or 7 to 9 16-CTA clusters at a time; admitting
 // more than that only queues kernels behind each other (measured: 94
 // concurrent 6480-unknown solves ran 4x slower in total than 16), so a request
 // that fits the memory budget still waits here until a solve finishes.

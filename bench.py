@@ -10,10 +10,10 @@ elements: 2160 boundary elements, NPG = 4, n = 6480 complex unknowns.  The
 per-mesh static work (GHMATECE) is done once before timing.
 
 Headline (`value`): the mixed+batched form, one step = one lockstep batch of
-`bem_sweep_batch_limit` frequency solves, 7 on this mesh (FP64 assembly,
-FP32 LU on TF32 tensor cores, FP64 iterative refinement), checked against
-the plain FP64 path at 1e-8.  The plain FP64 GPU path (one frequency at a
-time) is measured in the same run.
+`bem_sweep_batch_limit` frequency solves, 15 to 18 on this mesh as the device's
+GPCs hold clusters of 8 CTAs (FP64 assembly, FP32 LU on TF32 tensor cores, FP64
+iterative refinement), checked against the plain FP64 path at 1e-8.  The plain
+FP64 GPU path (one frequency at a time) is measured in the same run.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -538,6 +538,7 @@ def run_ours(args):
         "kernel_share": shares,
         "kernels": pm,
         "kernels_steps": max(3, args.steps // 2),
+        "kernels_note": "classes timed one by one on one lane, which turns lookahead off",
         "cuda_graphs": os.environ.get("BEM_GRAPHS", "1") != "0",
         "static_per_mesh": {"ghmatece_ms": round(static_ms, 3),
                             "kelvin_evals": s.nbe * (s.n - 1) * s.npg ** 2 + 4 * s.nbe * s.npg ** 2,
