@@ -133,8 +133,9 @@ def test_mixed_sweep_and_its_captured_step(nx, ny, refine):
     assert n > 10 and done >= 2  # the solves' tables, at least, are done without
 
 
-@pytest.mark.parametrize("form", ["plain", "mixed"])
-@pytest.mark.parametrize("nx,ny,count", [(9, 7, 5), (16, 15, 2)])
+# the last two sizes take lookahead, with buffers of its own
+@pytest.mark.parametrize("form,nx,ny,count", [("plain", 9, 7, 5), ("mixed", 9, 7, 5), ("plain", 16, 15, 2),
+                                              ("mixed", 16, 15, 2), ("plain", 25, 19, 2), ("mixed", 25, 19, 13)])
 def test_sweep_goes_on_with_fewer_problems(form, nx, ny, count):
     """Whichever buffer of a lockstep step finds no memory, the sweep runs in
     smaller steps and gives every solution."""
